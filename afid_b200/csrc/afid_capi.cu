@@ -82,6 +82,7 @@ struct Batch {
   FftSmem sm_y{0, 0}, sm_z{0, 0};   // slot and twiddle sizes of the persistent transforms
   int grid_y = 0, grid_z = 0;       // their resident grids
   int k2_block = 256;               // threads per block of the back-substitution kernel
+  int kseg = 0, nseg = 1;           // planes per block and blocks per column tile of the planewise marches
   size_t smem_wy[WY_NV] = {};       // shared memory and resident grids of the warp y transforms
   int grid_wy[WY_NV] = {};
   int grid_wz[WY_NV] = {};          // resident grids of the warp z transforms (shared memory as y)
@@ -492,6 +493,26 @@ int k2_block_size(const std::vector<BoxDev> &devs, int *out) {
   return 0;
 }
 
+int nsm_of_device() {
+  int dev = 0, nsm = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 148;
+  return nsm;
+}
+
+// Planes per block of the marches whose planes are independent (divergence,
+// correction, diagnostics), for a set of ``tiles`` column tiles and at most
+// nxm planes: whole columns once the tiles fill the resident blocks (two per
+// SM), else segments that give each SM two rounds of blocks.
+void plane_segments(int nsm, int tiles, int nxm, int *kseg, int *nseg) {
+  const long long resident = 2LL * nsm;
+  long long n = tiles >= resident ? 1 : cdiv(2 * resident, std::max(tiles, 1));
+  n = std::min(n, cdiv(nxm, KC_U));
+  *kseg = (int)(cdiv(cdiv(nxm, n), KC_U) * KC_U);
+  *nseg = (int)cdiv(nxm, *kseg);
+}
+
 int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split = true) {
   if (n <= 0 || !ids) return fail(AFID_EINVAL, "empty box set");
   std::vector<int> key(ids, ids + n);
@@ -550,6 +571,7 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
     off[(size_t)f * (n + 1) + n] = (int)acc;
     bt->total[f] = (int)acc;
   }
+  plane_segments(nsm_of_device(), bt->total[FAM_COL], devs[0].nxm, &bt->kseg, &bt->nseg);
   off.insert(off.end(), pos.begin(), pos.end());   // the positions follow the tile tables
   if (cudaMalloc(&bt->d_boxes, sizeof(BoxDev) * n) != cudaSuccess ||
       cudaMalloc(&bt->d_off, sizeof(int) * off.size()) != cudaSuccess) {
@@ -730,6 +752,26 @@ struct Prof {
     }                               \
   } while (0)
 
+// The marches with independent planes: whole columns, or segments of kseg
+// planes in a set whose column tiles do not fill the device (plane_segments).
+void launch_divergence(const Batch *bt, cudaStream_t s, int ns) {
+  const dim3 g(bt->total[FAM_COL], bt->nseg);
+  if (bt->nseg > 1) k_divergence<true><<<g, 256, 0, s>>>(bdev(bt, FAM_COL), ns, bt->kseg);
+  else k_divergence<false><<<g, 256, 0, s>>>(bdev(bt, FAM_COL), ns, 0);
+}
+
+void launch_correct(const Batch *bt, cudaStream_t s, int ns, int vel, int pr) {
+  const dim3 g(bt->total[FAM_COL], bt->nseg);
+  if (bt->nseg > 1) k_correct<true><<<g, 256, 0, s>>>(bdev(bt, FAM_COL), ns, vel, pr, bt->kseg);
+  else k_correct<false><<<g, 256, 0, s>>>(bdev(bt, FAM_COL), ns, vel, pr, 0);
+}
+
+void launch_diag(const Batch *bt, cudaStream_t s, int every_box) {
+  const dim3 g(bt->total[FAM_DIAG], bt->nseg);
+  if (bt->nseg > 1) k_diag<true><<<g, 256, 0, s>>>(bdev(bt, FAM_DIAG), every_box, bt->kseg);
+  else k_diag<false><<<g, 256, 0, s>>>(bdev(bt, FAM_DIAG), every_box, 0);
+}
+
 // The x-solve of the Poisson equation (total[f] tiles of family f; bd(f)
 // its descriptor).
 template <class BD>
@@ -743,7 +785,7 @@ int launch_poisson_x(const int *total, BD bd, cudaStream_t s, int ns) {
 
 int launch_poisson(const Batch *bt, cudaStream_t s, int ns, bool from_vel, Prof *pf = nullptr) {
   if (from_vel) {
-    k_divergence<<<bt->total[FAM_COL], 256, 0, s>>>(bdev(bt, FAM_COL), ns);
+    launch_divergence(bt, s, ns);
     CKL();
     PMARK(pf, AFID_K_DIVERGENCE);
   }
@@ -802,7 +844,7 @@ int launch_substep(const Batch *bt, cudaStream_t s, int ns, Prof *pf = nullptr) 
   PMARK(pf, AFID_K_IMPLICIT_BWD);
   int rc = launch_poisson(bt, s, ns, true, pf);
   if (rc) return rc;
-  k_correct<<<bt->total[FAM_COL], 256, 0, s>>>(bdev(bt, FAM_COL), ns, 1, 1);
+  launch_correct(bt, s, ns, 1, 1);
   CKL();
   PMARK(pf, AFID_K_CORRECT);
   return 0;
@@ -810,7 +852,7 @@ int launch_substep(const Batch *bt, cudaStream_t s, int ns, Prof *pf = nullptr) 
 
 int launch_step(const Batch *bt, cudaStream_t s, Prof *pf = nullptr) {
   const int nb = (int)bt->ids.size();
-  k_diag<<<bt->total[FAM_DIAG], 256, 0, s>>>(bdev(bt, FAM_DIAG), 0);
+  launch_diag(bt, s, 0);
   CKL();
   PMARK(pf, AFID_K_DIAG);
   k_finalize<<<cdiv(nb, 128), 128, 0, s>>>(bt->d_boxes, nb, 0);
@@ -1620,7 +1662,7 @@ int afid_calc_local_divergence(afid_ctx *c, int id) {
   Batch *bt;
   rc = single_batch(c, id, &bt);
   if (rc) return rc;
-  k_divergence<<<bt->total[FAM_COL], 256, 0, c->stream>>>(bdev(bt, FAM_COL), 0);
+  launch_divergence(bt, c->stream, 0);
   CKL();
   return 0;
 }
@@ -1642,7 +1684,7 @@ static int correct(afid_ctx *c, int id, int vel, int pr) {
   Batch *bt;
   rc = single_batch(c, id, &bt);
   if (rc) return rc;
-  k_correct<<<bt->total[FAM_COL], 256, 0, c->stream>>>(bdev(bt, FAM_COL), 0, vel, pr);
+  launch_correct(bt, c->stream, 0, vel, pr);
   CKL();
   return 0;
 }
@@ -1661,7 +1703,7 @@ static int diag_now(afid_ctx *c, int id, BoxScalars *bs) {
   if (rc) return rc;
   void *red = (char *)hb->dev.sc + offsetof(BoxScalars, red_u64);
   CK(cudaMemsetAsync(red, 0, sizeof(bs->red_u64), c->stream));
-  k_diag<<<bt->total[FAM_DIAG], 256, 0, c->stream>>>(bdev(bt, FAM_DIAG), 1);
+  launch_diag(bt, c->stream, 1);
   CKL();
   CK(cudaMemcpyAsync(bs, hb->dev.sc, sizeof(BoxScalars), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaMemsetAsync(red, 0, sizeof(bs->red_u64), c->stream));
