@@ -54,7 +54,7 @@ int fail(int code, const char *fmt, ...) {
 // lane), the others in FAM_FY; likewise the z transforms in FAM_WZ8/12 and
 // FAM_FZ.
 enum Fam { FAM_K1 = 0, FAM_COL, FAM_CELL, FAM_DIAG, FAM_FY, FAM_FZ, FAM_PX, FAM_K2,
-           FAM_WY8, FAM_WY12, FAM_WZ8, FAM_WZ12, NFAM };
+           FAM_WY8, FAM_WY12, FAM_WZ8, FAM_WZ12, FAM_K1S, FAM_KS, NFAM };
 constexpr int WY_NV = 2;
 constexpr int WY_V[WY_NV] = {8, 12};
 constexpr int HIST_CAP = 4096;
@@ -82,6 +82,8 @@ struct Batch {
   FftSmem sm_y{0, 0}, sm_z{0, 0};   // slot and twiddle sizes of the persistent transforms
   int grid_y = 0, grid_z = 0;       // their resident grids
   int k2_block = 256;               // threads per block of the back-substitution kernel
+  int k1s_seg = 0, k1s_nseg = 1;    // planes per block and blocks per tile of the K1 launch of the ks boxes
+  size_t smem_ks = 0;               // shared memory of k_implicit_cols
   int kseg = 0, nseg = 1;           // planes per block and blocks per column tile of the planewise marches
   size_t smem_wy[WY_NV] = {};       // shared memory and resident grids of the warp y transforms
   int grid_wy[WY_NV] = {};
@@ -185,14 +187,17 @@ int warp_plan(int n, int *v_out, int *g_out, int *rad, int *np, int min_g = 1) {
 //      block per SM at 128 registers)
 //   5: 32x4 tiles, 4 blocks/SM        6: 32x2 tiles, 8 blocks/SM
 //   7: 32x4 tiles, 5 blocks/SM        8: 32x4 tiles, 6 blocks/SM
+constexpr int KS_SMEM_MAX = 226 * 1024;   // of k_implicit_cols
 constexpr int K1_VMIN = 2, K1_VMAX = 8;
 constexpr int K1_DEFAULT = 4;   // the variant the tuner picks for the large boxes (768^2, 1280^2)
 int k1_tile_height(int variant) { return (variant == 5 || variant >= 7) ? 4 : variant == 6 ? 2 : 8; }
 
 long long tiles_of(const BoxDev &B, int fam, int k1_variant = 2, int k2_block = 256) {
   switch (fam) {
-    case FAM_K2: return cdiv(B.plane, k2_block);
-    case FAM_K1: return cdiv(B.nym, K1_TJ) * cdiv(B.nzm, k1_tile_height(k1_variant));
+    case FAM_K2: return B.on_chip ? 0 : cdiv(B.plane, k2_block);
+    case FAM_K1: return B.on_chip ? 0 : cdiv(B.nym, K1_TJ) * cdiv(B.nzm, k1_tile_height(k1_variant));
+    case FAM_K1S: return B.on_chip ? cdiv(B.nym, K1_TJ) * cdiv(B.nzm, 8) : 0;
+    case FAM_KS: return B.on_chip ? cdiv(B.plane, KS_COLS) : 0;
     case FAM_COL: return cdiv(B.plane, 256);
     case FAM_CELL: return cdiv((long long)B.nxm * B.plane, 256);
     case FAM_DIAG: return cdiv(B.plane, 256);
@@ -513,6 +518,38 @@ void plane_segments(int nsm, int tiles, int nxm, int *kseg, int *nseg) {
   *nseg = (int)cdiv(nxm, *kseg);
 }
 
+// Small sets (fewer than one block of 256 columns per SM) solve their implicit
+// systems on chip: K1 writes right-hand sides, k_implicit_cols does both
+// sweeps.  K1 + K2 per step: 75x150x135 (80 tiles) 0.48 -> 0.33 ms; twelve
+// ensemble boxes (about 330 tiles) 1.02 -> 1.12 ms, so the line lies between.
+// Boxes too tall for a block's shared memory (nxm > 401) keep the column
+// kernels.  Results do not depend on the choice.  Returns the shared memory of
+// the k_implicit_cols launch.
+size_t choose_on_chip(int nsm, std::vector<BoxDev> &devs) {
+  long long tiles = 0;
+  for (const BoxDev &d : devs) tiles += cdiv(d.plane, 256);
+  size_t smem = 0;
+  for (BoxDev &d : devs) {
+    d.on_chip = tiles < nsm && ks_bytes(d.nxm) <= KS_SMEM_MAX;
+    if (d.on_chip) smem = std::max(smem, (size_t)ks_bytes(d.nxm));
+  }
+  return smem;
+}
+
+// Planes per block of the K1 launch of such a set (one block per SM): the
+// number of segments with the least waves x (planes + the planes' worth of
+// time a block takes to fill its ring).
+void k1s_segments(int nsm, int tiles, int nxm, int *kseg, int *nseg) {
+  constexpr int FILL = 4;
+  long long best = -1;
+  *kseg = nxm;
+  *nseg = 1;
+  for (int ks = 2; ks < nxm + 2 && tiles > 0; ks += 2) {   // two planes per barrier
+    const long long n = cdiv(nxm, ks), cost = cdiv(tiles * n, nsm) * (ks + FILL);
+    if (best < 0 || cost < best) { best = cost; *kseg = ks; *nseg = (int)n; }
+  }
+}
+
 int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split = true) {
   if (n <= 0 || !ids) return fail(AFID_EINVAL, "empty box set");
   std::vector<int> key(ids, ids + n);
@@ -557,6 +594,8 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
     const char *e = getenv("AFID_K1_VARIANT");
     if (e && atoi(e) >= K1_VMIN && atoi(e) <= K1_VMAX) bt->k1_minb = atoi(e);
   }
+  const int nsm = nsm_of_device();
+  bt->smem_ks = choose_on_chip(nsm, devs);
   {
     int rc = k2_block_size(devs, &bt->k2_block);
     if (rc) { delete bt; return rc; }
@@ -571,7 +610,8 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
     off[(size_t)f * (n + 1) + n] = (int)acc;
     bt->total[f] = (int)acc;
   }
-  plane_segments(nsm_of_device(), bt->total[FAM_COL], devs[0].nxm, &bt->kseg, &bt->nseg);
+  plane_segments(nsm, bt->total[FAM_COL], devs[0].nxm, &bt->kseg, &bt->nseg);
+  k1s_segments(nsm, bt->total[FAM_K1S], devs[0].nxm, &bt->k1s_seg, &bt->k1s_nseg);
   off.insert(off.end(), pos.begin(), pos.end());   // the positions follow the tile tables
   if (cudaMalloc(&bt->d_boxes, sizeof(BoxDev) * n) != cudaSuccess ||
       cudaMalloc(&bt->d_off, sizeof(int) * off.size()) != cudaSuccess) {
@@ -703,13 +743,15 @@ int init_kernel_attrs() {
   CK(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return fail(AFID_EINVAL, "device %d out of range", dev);
   if (done[dev]) return 0;
-  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 8>::SMEM));
-  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 8>::SMEM));
-  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<2, 8>::SMEM));
-  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<4, 4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 4>::SMEM));
-  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<2, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 2>::SMEM));
-  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<4, 5, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 4>::SMEM));
-  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<4, 6, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 4>::SMEM));
+  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 2, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 8>::SMEM));
+  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 3, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 8>::SMEM));
+  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 2, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<2, 8>::SMEM));
+  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<2, 8>::SMEM));
+  CK(cudaFuncSetAttribute(k_implicit_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, KS_SMEM_MAX));
+  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<4, 4, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 4>::SMEM));
+  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<2, 8, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 2>::SMEM));
+  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<4, 5, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 4>::SMEM));
+  CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<4, 6, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 4>::SMEM));
   const int fsm = FFT_SMEM_MAX;   // two slots + work + twiddles: (4 N + 4) 16 bytes at one line
   CK(cudaFuncSetAttribute(k_fft_y_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
   CK(cudaFuncSetAttribute(k_fft_y_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
@@ -828,18 +870,22 @@ int launch_substep(const Batch *bt, cudaStream_t s, int ns, Prof *pf = nullptr) 
   PMARK(pf, AFID_K_PREP);
   const BatchDev k1 = bdev(bt, FAM_K1);
   const int nk1 = bt->total[FAM_K1];
-  switch (bt->k1_minb) {
-    case 3: k_explicit_implicit_fwd<8, 3, 1><<<nk1, 256, K1Ring<1, 8>::SMEM, s>>>(k1, ns); break;
-    case 4: k_explicit_implicit_fwd<8, 2, 2><<<nk1, 256, K1Ring<2, 8>::SMEM, s>>>(k1, ns); break;
-    case 5: k_explicit_implicit_fwd<4, 4, 1><<<nk1, 128, K1Ring<1, 4>::SMEM, s>>>(k1, ns); break;
-    case 6: k_explicit_implicit_fwd<2, 8, 1><<<nk1, 64, K1Ring<1, 2>::SMEM, s>>>(k1, ns); break;
-    case 7: k_explicit_implicit_fwd<4, 5, 1><<<nk1, 128, K1Ring<1, 4>::SMEM, s>>>(k1, ns); break;
-    case 8: k_explicit_implicit_fwd<4, 6, 1><<<nk1, 128, K1Ring<1, 4>::SMEM, s>>>(k1, ns); break;
-    default: k_explicit_implicit_fwd<8, 2, 1><<<nk1, 256, K1Ring<1, 8>::SMEM, s>>>(k1, ns); break;
+  if (nk1) switch (bt->k1_minb) {
+    case 3: k_explicit_implicit_fwd<8, 3, 1, false><<<nk1, 256, K1Ring<1, 8>::SMEM, s>>>(k1, ns, 0); break;
+    case 4: k_explicit_implicit_fwd<8, 2, 2, false><<<nk1, 256, K1Ring<2, 8>::SMEM, s>>>(k1, ns, 0); break;
+    case 5: k_explicit_implicit_fwd<4, 4, 1, false><<<nk1, 128, K1Ring<1, 4>::SMEM, s>>>(k1, ns, 0); break;
+    case 6: k_explicit_implicit_fwd<2, 8, 1, false><<<nk1, 64, K1Ring<1, 2>::SMEM, s>>>(k1, ns, 0); break;
+    case 7: k_explicit_implicit_fwd<4, 5, 1, false><<<nk1, 128, K1Ring<1, 4>::SMEM, s>>>(k1, ns, 0); break;
+    case 8: k_explicit_implicit_fwd<4, 6, 1, false><<<nk1, 128, K1Ring<1, 4>::SMEM, s>>>(k1, ns, 0); break;
+    default: k_explicit_implicit_fwd<8, 2, 1, false><<<nk1, 256, K1Ring<1, 8>::SMEM, s>>>(k1, ns, 0); break;
   }
+  if (bt->total[FAM_K1S])
+    k_explicit_implicit_fwd<8, 2, 2, true><<<dim3(bt->total[FAM_K1S], bt->k1s_nseg), 256, K1Ring<2, 8>::SMEM, s>>>(
+        bdev(bt, FAM_K1S), ns, bt->k1s_seg);
   CKL();
   PMARK(pf, AFID_K_EXPLICIT_FWD);
-  k_implicit_bwd<<<bt->total[FAM_K2], bt->k2_block, 0, s>>>(bdev(bt, FAM_K2), ns);
+  if (bt->total[FAM_K2]) k_implicit_bwd<<<bt->total[FAM_K2], bt->k2_block, 0, s>>>(bdev(bt, FAM_K2), ns);
+  if (bt->total[FAM_KS]) k_implicit_cols<<<dim3(bt->total[FAM_KS], 2), 64, bt->smem_ks, s>>>(bdev(bt, FAM_KS), ns);
   CKL();
   PMARK(pf, AFID_K_IMPLICIT_BWD);
   int rc = launch_poisson(bt, s, ns, true, pf);

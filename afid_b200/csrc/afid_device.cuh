@@ -59,10 +59,10 @@ enum TabId {
 
 // Per-substep tridiagonal tables in BoxDev::coef: for system s in
 // {SYS_X (vx, size nx), SYS_YZ (vy/vz, size nxm), SYS_T (temp, size nx)}
-// the arrays (sc, fact, dp, du, g) each of length nx at
-// coef[(s * C_N + a) * nx + k].
+// the arrays (sc, fact, dp, du, g, rd, ud) each of length nx at
+// coef[(s * C_N + a) * nx + k]; rd = 1/dp and ud = du/dp.
 enum SysId { SYS_X = 0, SYS_YZ = 1, SYS_T = 2, SYS_N = 3 };
-enum CoefId { C_SC = 0, C_FACT, C_DP, C_DU, C_G, C_N };
+enum CoefId { C_SC = 0, C_FACT, C_DP, C_DU, C_G, C_RD, C_UD, C_N };
 
 constexpr int HIST_FIELDS = 8;   // time, dt, cfl_used, divmax, nu_bot, nu_top, vmax_y, vmax_z
 
@@ -99,7 +99,7 @@ struct BoxDev {
   double *nu_part;      // per-block partial sums of the plate Nu reduction
   double *hist;         // per-step records, HIST_FIELDS doubles each (ring)
   int hist_cap;
-  int pad1_;
+  int on_chip;          // 1: the x-solves of a small set (k_implicit_cols), 0: k_implicit_bwd
   BoxScalars *sc;
   int fft_y_radix[16];  // radices of nym (Stockham passes), terminated by 0
   int fft_z_radix[16];  // radices of nzm

@@ -126,6 +126,16 @@ __device__ __forceinline__ double rhs_temp(double H, double Hold, double tp, dou
   return (ga * H + ro * Hold + alpec * dxx) * dt;
 }
 
+// One row of the forward elimination and of the back substitution of the
+// fused x-solves (dgttrs with the pivots' reciprocals): y = bb - fact y(k-1),
+// x = (y - du x(k+1)) / dp as y rd - ud x(k+1), so that the serial chain of a
+// column is one multiply-add per row.  Every fused kernel goes through these,
+// so a box's result does not depend on which of them run it.
+__device__ __forceinline__ double fwd_row(double bb, double fact, double y) { return __fma_rn(-fact, y, bb); }
+__device__ __forceinline__ double bwd_row(double y, double rd, double ud, double x) {
+  return __fma_rn(-ud, x, y * rd);
+}
+
 __device__ __forceinline__ const double *coefp(const BoxDev &B, int sys, int arr) {
   return B.coef + (long long)(sys * C_N + arr) * B.nx;
 }
@@ -224,6 +234,14 @@ __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int n
     for (int k = n; k < nx; ++k) { dl[k] = 0.0; dp[k] = 1.0; g[k] = 0.0; }
     if (pivot_needed) atomicExch(&S->status, -2);
   }
+  __syncthreads();
+  for (int t = threadIdx.x; t < 3 * nx; t += blockDim.x) {
+    const int sys = t / nx, k = t % nx;
+    double *c = B.coef + (long long)(sys * C_N) * nx + k;
+    const double rd = 1.0 / c[(long long)C_DP * nx];
+    c[(long long)C_RD * nx] = rd;
+    c[(long long)C_UD * nx] = c[(long long)C_DU * nx] * rd;
+  }
 }
 
 constexpr int K1_TJ = 32;                       // tile width along y (one warp)
@@ -318,8 +336,15 @@ struct K1Ring {
   static constexpr int SMEM = (NS * F_NF * K1Shape<TI>::PL + NS * 16 + NS * HS) * 8;
 };
 
-template <int TI, int MINB, int PPB>
-__global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd(BatchDev bt, int ns) {
+//
+// RHS: sets whose x-solves run in k_implicit_cols.  The scaled right-hand
+// sides are written instead of the forward vectors (the first row of vx, which
+// the carried wall row enters, is its forward vector already), so planes do
+// not depend on each other and block (tile, s) marches the planes s kseg ..
+// only: one march of all planes took 67 us on 65x64x64 (16 tiles on 148 SMs),
+// segments of 8 planes 18 us.
+template <int TI, int MINB, int PPB, bool RHS>
+__global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd(BatchDev bt, int ns, int kseg) {
   constexpr int NS = K1Ring<PPB, TI>::NS;
   constexpr int D = K1Ring<PPB, TI>::D;
   constexpr int PL = K1Shape<TI>::PL, NT = K1Shape<TI>::NT, NLD = K1Shape<TI>::NLD;
@@ -333,6 +358,9 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
   if (!B.active || ns >= B.nsst) return;
   const BoxScalars *S = B.sc;
   if (S->status != 0) return;
+  const int ks = RHS ? (int)blockIdx.y * kseg : 0;   // planes [ks, ke) of this block
+  const int ke = RHS ? min(ks + kseg, B.nxm) : B.nxm;
+  if (RHS && ks >= ke) return;
   const int tid = threadIdx.x;
   const int tile = blockIdx.x - __ldg(bt.tile_off + b);
   const int nym = B.nym, nzm = B.nzm;
@@ -386,7 +414,7 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
     hdst[q] = fq * NT + hrow * K1_TJ + hj;
   }
   auto load_plane = [&](int p) {      // plane p and its per-k scalars into slot p % NS
-    if (p > nx - 1) return;
+    if (p > (RHS ? ke : nx - 1)) return;
     const int sl = p % NS;
     double *dst = ring + sl * F_NF * PL;
     const long long po = (long long)p * P;
@@ -414,24 +442,30 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
   acc.prev = K1Prev{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
 
   // forward-sweep carries
-  double yX = inside ? B.wall[col] : 0.0;   // rhs(1,j,i) left by the last vz solve
+  double yX = inside && ks == 0 ? B.wall[col] : 0.0;   // rhs(1,j,i) left by the last vz solve
   double yY = 0.0, yZ = 0.0, yT = 0.0;
 
-  for (int p = 0; p < D - PPB; ++p) load_plane(p);
+  for (int p = 0; p < D - PPB; ++p) load_plane(ks + p);
   cp_async_commit();
-  for (int p = D - PPB; p < D; ++p) load_plane(p);
+  for (int p = D - PPB; p < D; ++p) load_plane(ks + p);
   cp_async_commit();
+  if (RHS && ks > 0 && inside) {   // plane ks - 1 of this column
+    const long long o = (long long)(ks - 1) * P + col;
+    const long long ojp = (j == nym - 1 ? 1 - nym : 1), oip = (i == nzm - 1 ? (long long)(1 - nzm) * nym : nym);
+    acc.prev = K1Prev{fld[F_VX][o], fld[F_VY][o], fld[F_VY][o + ojp], fld[F_VZ][o], fld[F_VZ][o + oip], fld[F_T][o],
+                      fld[F_PR][o]};
+  }
   cp_async_wait_1();
   __syncthreads();
 
-  for (int k0 = 0; k0 < nxm; k0 += PPB) {
+  for (int k0 = ks; k0 < ke; k0 += PPB) {
 #pragma unroll
     for (int u = 0; u < PPB; ++u) load_plane(k0 + D + u);
     cp_async_commit();
 #pragma unroll
     for (int u = 0; u < PPB; ++u) {
       const int kc = k0 + u;
-      if (kc >= nxm) break;
+      if (kc >= ke) break;
       acc.s_c = kc % NS;
       acc.s_p = (kc + 1) % NS;
       const double *tk = tring + (kc % NS) * 16;
@@ -450,7 +484,7 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
                                    acc(F_VY, dkm, 0, 0), am_s, ac_s, ap_s, dyp, ga, ro, alre, dt);
           __stwb(ruy + o, H);
           const double bb = r * tk[KT_YSC];
-          yY = (kc == 0) ? bb : bb - tk[KT_YF] * yY;
+          yY = RHS || kc == 0 ? bb : fwd_row(bb, tk[KT_YF], yY);
           __stwb(yb1 + o, yY);
         }
         {
@@ -460,7 +494,7 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
                                    acc(F_VZ, dkm, 0, 0), am_s, ac_s, ap_s, dzp, ga, ro, alre, dt);
           __stwb(ruz + o, H);
           const double bb = r * tk[KT_YSC];
-          yZ = (kc == 0) ? bb : bb - tk[KT_YF] * yZ;
+          yZ = RHS || kc == 0 ? bb : fwd_row(bb, tk[KT_YF], yZ);
           __stwb(yb2 + o, yZ);
         }
         if (kc >= 1) {
@@ -473,7 +507,7 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
                                     am_c, ac_c, ap_c, al, ga, ro, alre, dt, udx3c_k);
             __stwb(rux + o, H);
             const double bb = r * tk[KT_XSC];
-            yX = bb - tk[KT_XF] * yX;
+            yX = RHS && kc > 1 ? bb : fwd_row(bb, tk[KT_XF], yX);
             __stwb(yb0 + o, yX);
           }
           {
@@ -482,7 +516,7 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
                                       acc(F_T, -1, 0, 0), am_c, ac_c, ap_c, ga, ro, alpec, dt);
             __stwb(rut + o, H);
             const double bb = r * tk[KT_TSC];
-            yT = bb - tk[KT_TF] * yT;
+            yT = RHS ? bb : fwd_row(bb, tk[KT_TF], yT);
             __stwb(yb3 + o, yT);
           }
         }
@@ -548,19 +582,13 @@ __global__ void __launch_bounds__(256, 3) k_implicit_bwd(BatchDev bt, int ns) {
       const int k = k0 - u;
       if (k < 0) break;
       const long long o = (long long)k * P;
-      const double dy_ = lu(SYS_YZ, C_DP, k);
-      if (k == nxm - 1) {
-        xY = a1[u] / dy_;
-        xZ = a2[u] / dy_;
-      } else {
-        const double uu = lu(SYS_YZ, C_DU, k);
-        xY = (a1[u] - uu * xY) / dy_;
-        xZ = (a2[u] - uu * xZ) / dy_;
-      }
+      const double rd = lu(SYS_YZ, C_RD, k), ud = lu(SYS_YZ, C_UD, k);
+      xY = bwd_row(a1[u], rd, ud, xY);
+      xZ = bwd_row(a2[u], rd, ud, xZ);
       vy[o] = q1[u] + xY;
       vz[o] = q2[u] + xZ;
       if (k >= 1) {
-        xX = (a0[u] - lu(SYS_X, C_DU, k) * xX) / lu(SYS_X, C_DP, k);
+        xX = bwd_row(a0[u], lu(SYS_X, C_RD, k), lu(SYS_X, C_UD, k), xX);
         vx[o] = q0[u] + xX;
       }
     }
@@ -582,13 +610,131 @@ __global__ void __launch_bounds__(256, 3) k_implicit_bwd(BatchDev bt, int ns) {
     for (int u = 0; u < K2_U; ++u) {
       const int k = k0 - u;
       if (k < 1) break;
-      const double y = a3[u] + lu(SYS_T, C_G, k) * w;
-      xT = (y - lu(SYS_T, C_DU, k) * xT) / lu(SYS_T, C_DP, k);
+      const double y = __fma_rn(lu(SYS_T, C_G, k), w, a3[u]);
+      xT = bwd_row(y, lu(SYS_T, C_RD, k), lu(SYS_T, C_UD, k), xT);
       tp[(long long)k * P] = q3[u] + xT;
     }
   }
   tp[0] = B.tempbp;
   tp[(long long)(nx - 1) * P] = B.temptp;
+}
+
+// ---------------------------------------------------------------------------
+// K2 of small sets: forward elimination, back substitution and update from
+// the right-hand sides K1 wrote, with the columns on chip.  A block takes 32
+// neighbouring columns of two fields: vx and vy (blockIdx.y = 0) or vz and temp
+// (1).  Warp w solves one field, a lane one column, its rows in the warp's part
+// of shared memory.  All rows are copied in at once (cp.async, 16 bytes a
+// lane), so a column costs one load latency instead of one per chunk of
+// planes, and the updated field is read KS_U planes ahead of the back
+// substitution.  The temperature's back substitution waits for the wall value
+// of the vz solve.  K2 of a 65x64x64 box: 54 us as k_implicit_bwd, 18 us here
+// (whose chain is one multiply-add and a shared-memory access per row).  In
+// sets that fill the SMs the few warps per SM cannot keep HBM busy (64-box
+// ensemble 2.3 ms per step against 1.3), so those keep k_implicit_bwd.
+// ---------------------------------------------------------------------------
+constexpr int KS_COLS = 32;      // columns per block
+constexpr int KS_U = 8;          // rows read ahead of the sweeps
+// shared memory of a block: 2 fields x nxm x 32 values, and per field the
+// rows' coefficients (fact, g, rd, ud), read broadcast
+__host__ __device__ constexpr int ks_bytes(int nxm) { return 2 * nxm * (KS_COLS + 4) * 8; }
+
+// the barrier of the vz and temp warps, reached at different places
+__device__ __forceinline__ void ks_barrier() { asm volatile("bar.sync 1, 64;\n" ::: "memory"); }
+
+__global__ void __launch_bounds__(64) k_implicit_cols(BatchDev bt, int ns) {
+  extern __shared__ double ksm[];
+  __shared__ double ws[KS_COLS];
+  const int b = find_box(bt.tile_off, bt.nbox, blockIdx.x);
+  const BoxDev &B = bt.boxes[b];
+  if (!B.active || ns >= B.nsst) return;
+  if (B.sc->status != 0) return;
+  const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int f = 2 * blockIdx.y + wp;           // 0 vx, 1 vy, 2 vz, 3 temp
+  const int nx = B.nx, nxm = B.nxm;
+  const long long P = B.plane;
+  const long long c0 = (long long)(blockIdx.x - __ldg(bt.tile_off + b)) * KS_COLS;
+  const bool node = f == 0 || f == 3;          // rows 1..nxm-1 of size nx, else 0..nxm-1
+  const int kb = node ? 1 : 0;
+  const int sys = f == 0 ? SYS_X : f == 3 ? SYS_T : SYS_YZ;
+  const double *__restrict__ src = B.ybuf[f];
+  double *__restrict__ q = f == 0 ? B.vx : f == 1 ? B.vy : f == 2 ? B.vz : B.temp;
+  double2 *const tab = reinterpret_cast<double2 *>(ksm) + 2 * wp * nxm;   // row k: (fact, g), (rd, ud)
+  double *const rows = ksm + 8 * nxm + wp * nxm * KS_COLS;
+  for (int k = lane; k < nxm; k += 32) {
+    double *const t = reinterpret_cast<double *>(tab + 2 * k);
+    cp_async8(t, coefp(B, sys, C_FACT) + k);
+    cp_async8(t + 1, coefp(B, sys, C_G) + k);
+    cp_async8(t + 2, coefp(B, sys, C_RD) + k);
+    cp_async8(t + 3, coefp(B, sys, C_UD) + k);
+  }
+  {
+    const int p2 = 2 * (lane & 15);            // a pair of columns is inside the plane or outside (P is even)
+    if (c0 + p2 < P)
+      for (int k = kb + (lane >> 4); k < nxm; k += 2)
+        cp_async16(rows + k * KS_COLS + p2, src + (long long)k * P + c0 + p2);
+  }
+  cp_async_commit();
+  const long long col = c0 + lane;
+  const bool ok = col < P;
+  double *const qc = q + (ok ? col : 0);
+  double qa[KS_U];
+#pragma unroll
+  for (int u = 0; u < KS_U; ++u) qa[u] = nxm - 1 - u >= kb ? qc[(long long)(nxm - 1 - u) * P] : 0.0;
+  cp_async_wait_all();
+  __syncwarp();
+  double *const s = rows + lane;
+  double y = node ? 0.0 : s[0];
+  for (int k0 = 1; k0 < nxm; k0 += KS_U) {
+    double r[KS_U], fk[KS_U];
+#pragma unroll
+    for (int u = 0; u < KS_U; ++u) {
+      const int k = min(k0 + u, nxm - 1);
+      r[u] = s[k * KS_COLS];
+      fk[u] = tab[2 * k].x;
+    }
+#pragma unroll
+    for (int u = 0; u < KS_U; ++u) {
+      if (k0 + u >= nxm) break;
+      y = fwd_row(r[u], fk[u], y);
+      s[(k0 + u) * KS_COLS] = y;
+    }
+  }
+  if (f == 3) ks_barrier();
+  const double w = f == 3 ? ws[lane] : 0.0;
+  double x = 0.0;
+  for (int k0 = nxm - 1; k0 >= kb; k0 -= KS_U) {
+    double qn[KS_U], r[KS_U];
+    double2 t[KS_U];
+#pragma unroll
+    for (int u = 0; u < KS_U; ++u) {
+      const int k = k0 - KS_U - u;
+      qn[u] = k >= kb ? qc[(long long)k * P] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < KS_U; ++u) {
+      const int k = max(k0 - u, kb);
+      r[u] = s[k * KS_COLS];
+      t[u] = tab[2 * k + 1];
+      if (f == 3) r[u] = __fma_rn(tab[2 * k].y, w, r[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < KS_U; ++u) {
+      const int k = k0 - u;
+      if (k < kb) break;
+      x = bwd_row(r[u], t[u].x, t[u].y, x);
+      if (ok) qc[(long long)k * P] = qa[u] + x;
+    }
+#pragma unroll
+    for (int u = 0; u < KS_U; ++u) qa[u] = qn[u];
+  }
+  if (f == 2) {
+    ws[lane] = x;
+    ks_barrier();
+    if (ok) B.wall[col] = x;                   // rhs(1,j,i) after the vz solve
+  }
+  if (ok && f == 0) { qc[0] = 0.0; qc[(long long)(nx - 1) * P] = 0.0; }
+  if (ok && f == 3) { qc[0] = B.tempbp; qc[(long long)(nx - 1) * P] = B.temptp; }
 }
 
 // ---------------------------------------------------------------------------

@@ -2,11 +2,15 @@
 columns in launches that fill the device and segments of planes in small
 ones.  Both forms against the oracle, bit for bit: segments with a last
 segment of 1, 2, 3 and 4 planes, and one box whose column tiles are enough for
-whole columns (288 x 270 columns)."""
+whole columns (288 x 270 columns).
+
+The implicit solves of a small set run on chip from right-hand sides
+(k_implicit_cols), those of a set that fills the device as column sweeps; a
+box's result is the same bits either way."""
 import numpy as np
 import pytest
 
-from helpers import cfg_of, oracle_state
+from helpers import cfg_of, compare_fields, oracle_state, FIELDS
 from oracle import afid_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -36,4 +40,49 @@ def test_planewise_marches_match_oracle(ctx, nxm, nym, nzm):
     O.correct_pressure(s, al, cfg.dt / s.p.ren * 0.5)
     for f in ("vx", "vy", "vz", "pr"):
         assert np.array_equal(box.download(f)[:nxm], getattr(s, f)[:nxm]), f
+    ctx.remove_box(box)
+
+
+def _boxes(ctx, cfgs):
+    out = []
+    for q, cfg in enumerate(cfgs):
+        s = oracle_state(cfg, seed=20 + q)
+        box = ctx.add_box(cfg, s.g.xc)
+        for f in FIELDS:
+            box.upload(f, getattr(s, f))
+        out.append(box)
+    return out
+
+
+@pytest.mark.parametrize("k1", [0, 2, 3, 5, 6, 7, 8])
+def test_on_chip_and_column_solves_agree(ctx, k1):
+    cfgs = [cfg_of(19, 30, 45, dt=5e-4, ylen=1.2, zlen=1.8), cfg_of(18, 16, 12, dt=5e-4, inslws=0),
+            cfg_of(41, 64, 36, dt=5e-4, nsst=1)]
+    filler = cfg_of(6, 200, 200, dt=1e-4)      # 157 tiles of 256 columns: the set fills the device
+    alone = _boxes(ctx, cfgs)
+    for b in alone:
+        ctx.step([b], 3)
+    batch = _boxes(ctx, cfgs + [filler])
+    for b in batch:
+        b.set_tuning(0, 0, k1)
+    ctx.step(batch, 3)
+    for a, b in zip(alone, batch):
+        for f in FIELDS + ("rux", "ruy", "ruz", "rutemp", "wall"):
+            assert np.array_equal(a.download(f), b.download(f)), f
+    for b in alone + batch:
+        ctx.remove_box(b)
+
+
+@pytest.mark.parametrize("nxm", [4, 9, 33, 400, 404])
+def test_on_chip_solves_match_oracle(ctx, nxm):
+    """nxm = 400 is near the tallest on-chip column, 404 is beyond it."""
+    cfg = cfg_of(nxm, 10, 12, dt=5e-4, ray=1e6, ylen=0.9, zlen=1.1, istr3=0 if nxm > 300 else 7)
+    s = oracle_state(cfg, seed=6)
+    box = ctx.add_box(cfg, s.g.xc)
+    for f in FIELDS:
+        box.upload(f, getattr(s, f))
+    O.run(s, 2, cfg.dt)
+    ctx.step([box], 2)
+    err = compare_fields(box, s)
+    assert all(v <= 1e-11 for v in err.values()), err
     ctx.remove_box(box)
