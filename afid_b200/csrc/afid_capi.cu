@@ -54,7 +54,7 @@ int fail(int code, const char *fmt, ...) {
 // lane), the others in FAM_FY; likewise the z transforms in FAM_WZ8/12 and
 // FAM_FZ.
 enum Fam { FAM_K1 = 0, FAM_COL, FAM_CELL, FAM_DIAG, FAM_FY, FAM_FZ, FAM_PX, FAM_K2,
-           FAM_WY8, FAM_WY12, FAM_WZ8, FAM_WZ12, FAM_K1S, FAM_KS, NFAM };
+           FAM_WY8, FAM_WY12, FAM_WZ8, FAM_WZ12, FAM_K1S, FAM_KS, FAM_PXS, NFAM };
 constexpr int WY_NV = 2;
 constexpr int WY_V[WY_NV] = {8, 12};
 constexpr int HIST_CAP = 4096;
@@ -84,6 +84,7 @@ struct Batch {
   int k2_block = 256;               // threads per block of the back-substitution kernel
   int k1s_seg = 0, k1s_nseg = 1;    // planes per block and blocks per tile of the K1 launch of the ks boxes
   size_t smem_ks = 0;               // shared memory of k_implicit_cols
+  size_t smem_px = 0;               // shared memory of k_poisson_cols (0: the set runs k_poisson_x)
   int kseg = 0, nseg = 1;           // planes per block and blocks per column tile of the planewise marches
   size_t smem_wy[WY_NV] = {};       // shared memory and resident grids of the warp y transforms
   int grid_wy[WY_NV] = {};
@@ -187,7 +188,7 @@ int warp_plan(int n, int *v_out, int *g_out, int *rad, int *np, int min_g = 1) {
 //      block per SM at 128 registers)
 //   5: 32x4 tiles, 4 blocks/SM        6: 32x2 tiles, 8 blocks/SM
 //   7: 32x4 tiles, 5 blocks/SM        8: 32x4 tiles, 6 blocks/SM
-constexpr int KS_SMEM_MAX = 226 * 1024;   // of k_implicit_cols
+constexpr int ON_CHIP_SMEM = 226 * 1024;   // most shared memory of k_implicit_cols and k_poisson_cols
 constexpr int K1_VMIN = 2, K1_VMAX = 8;
 constexpr int K1_DEFAULT = 4;   // the variant the tuner picks for the large boxes (768^2, 1280^2)
 int k1_tile_height(int variant) { return (variant == 5 || variant >= 7) ? 4 : variant == 6 ? 2 : 8; }
@@ -208,6 +209,7 @@ long long tiles_of(const BoxDev &B, int fam, int k1_variant = 2, int k2_block = 
     case FAM_WZ8: case FAM_WZ12:
       return B.wz_v == WY_V[fam - FAM_WZ8] ? (long long)B.nxm * wz_units_per_plane(B) : 0;
     case FAM_PX: return cdiv(px_pairs(B.nzm, B.nymh), 256);
+    case FAM_PXS: return cdiv((long long)B.nzm * B.nymh, 32);
   }
   return 0;
 }
@@ -530,10 +532,24 @@ size_t choose_on_chip(int nsm, std::vector<BoxDev> &devs) {
   for (const BoxDev &d : devs) tiles += cdiv(d.plane, 256);
   size_t smem = 0;
   for (BoxDev &d : devs) {
-    d.on_chip = tiles < nsm && ks_bytes(d.nxm) <= KS_SMEM_MAX;
+    d.on_chip = tiles < nsm && ks_bytes(d.nxm) <= ON_CHIP_SMEM;
     if (d.on_chip) smem = std::max(smem, (size_t)ks_bytes(d.nxm));
   }
   return smem;
+}
+
+// Shared memory of the on-chip x-solve (k_poisson_cols) for a set of ``warps``
+// groups of 32 modes and at most nxm planes, or 0 for k_poisson_x: on chip up
+// to four rounds of the warps the SMs hold, in a half of a split set (whose
+// other half runs beside it) up to two.  Per step, on chip against k_poisson_x:
+// 65x64x64 (0.1 rounds) 0.042 and 0.129 ms, 48x384x243 (1.1) 0.081 and 0.123,
+// twelve ensemble boxes (2.4) 0.123 and 0.223, 24 (4.1) 0.227 and 0.279, 64
+// (11) 0.497 and 0.492, 192x384x384 (7.8) 0.80 and 0.61; whole steps of split
+// sets, 20 boxes (halves of 1.8 rounds) 3.24 and 3.32, 24 (2.0) 3.75 and 3.64.
+size_t px_cols_smem(int nsm, int warps, int nxm, bool half) {
+  const int bytes = px_cols_bytes(nxm);
+  if (bytes > ON_CHIP_SMEM) return 0;
+  return warps <= (half ? 2LL : 4LL) * nsm * (ON_CHIP_SMEM / bytes) ? (size_t)bytes : 0;
 }
 
 // Planes per block of the K1 launch of such a set (one block per SM): the
@@ -610,6 +626,7 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
     off[(size_t)f * (n + 1) + n] = (int)acc;
     bt->total[f] = (int)acc;
   }
+  bt->smem_px = px_cols_smem(nsm, bt->total[FAM_PXS], devs[0].nxm, !allow_split);
   plane_segments(nsm, bt->total[FAM_COL], devs[0].nxm, &bt->kseg, &bt->nseg);
   k1s_segments(nsm, bt->total[FAM_K1S], devs[0].nxm, &bt->k1s_seg, &bt->k1s_nseg);
   off.insert(off.end(), pos.begin(), pos.end());   // the positions follow the tile tables
@@ -747,7 +764,8 @@ int init_kernel_attrs() {
   CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 3, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 8>::SMEM));
   CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 2, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<2, 8>::SMEM));
   CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<8, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<2, 8>::SMEM));
-  CK(cudaFuncSetAttribute(k_implicit_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, KS_SMEM_MAX));
+  CK(cudaFuncSetAttribute(k_poisson_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, ON_CHIP_SMEM));
+  CK(cudaFuncSetAttribute(k_implicit_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, ON_CHIP_SMEM));
   CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<4, 4, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 4>::SMEM));
   CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<2, 8, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 2>::SMEM));
   CK(cudaFuncSetAttribute(k_explicit_implicit_fwd<4, 5, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, K1Ring<1, 4>::SMEM));
@@ -817,8 +835,11 @@ void launch_diag(const Batch *bt, cudaStream_t s, int every_box) {
 // The x-solve of the Poisson equation (total[f] tiles of family f; bd(f)
 // its descriptor).
 template <class BD>
-int launch_poisson_x(const int *total, BD bd, cudaStream_t s, int ns) {
-  if (total[FAM_PX] > 0) {
+int launch_poisson_x(const int *total, BD bd, size_t smem_cols, cudaStream_t s, int ns) {
+  if (smem_cols) {
+    k_poisson_cols<<<total[FAM_PXS], 32, smem_cols, s>>>(bd(FAM_PXS), ns);
+    CKL();
+  } else if (total[FAM_PX] > 0) {
     k_poisson_x<<<total[FAM_PX], 256, 0, s>>>(bd(FAM_PX), ns);
     CKL();
   }
@@ -844,7 +865,7 @@ int launch_poisson(const Batch *bt, cudaStream_t s, int ns, bool from_vel, Prof 
   }
   PMARK(pf, AFID_K_FFT_Z_FWD);
   {
-    int rc = launch_poisson_x(bt->total, [&](int fam) { return bdev(bt, fam); }, s, ns);
+    int rc = launch_poisson_x(bt->total, [&](int fam) { return bdev(bt, fam); }, bt->smem_px, s, ns);
     if (rc) return rc;
   }
   PMARK(pf, AFID_K_POISSON_X);
@@ -2335,7 +2356,7 @@ extern "C" int afid_solve_pressure_correction_noalloc(double *dph, int nxm, int 
   static_assert(sizeof(off) <= 16 * sizeof(double), "tile tables exceed their scratch slot");
   for (int f = 0; f < NFAM; ++f) {
     off[f][0] = 0;
-    off[f][1] = total[f] = (f == FAM_FY || f == FAM_FZ || f == FAM_PX || f >= FAM_WY8) ? (int)tiles_of(d, f) : 0;
+    off[f][1] = total[f] = (f == FAM_FY || f == FAM_FZ || f == FAM_PX || f == FAM_PXS || (f >= FAM_WY8 && f <= FAM_WZ12)) ? (int)tiles_of(d, f) : 0;
   }
   CK(cudaMemcpyAsync(base + o_tab, tab, (size_t)n_tab * 8, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(base + o_tw, g_noalloc_host.tw, (size_t)(nym + nzm) * 16, cudaMemcpyHostToDevice, st));
@@ -2364,7 +2385,7 @@ extern "C" int afid_solve_pressure_correction_noalloc(double *dph, int nxm, int 
   if (rc) return rc;
   rc = launch_fft_z<-1>(total, bd, gz, sz, smz, gwz, swy, st, 0);
   if (rc) return rc;
-  rc = launch_poisson_x(total, bd, st, 0);
+  rc = launch_poisson_x(total, bd, px_cols_smem(nsm_of_device(), total[FAM_PXS], nxm, false), st, 0);
   if (rc) return rc;
   rc = launch_fft_z<+1>(total, bd, gz, sz, smz, gwz, swy, st, 0);
   if (rc) return rc;

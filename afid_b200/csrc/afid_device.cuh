@@ -86,8 +86,8 @@ struct BoxDev {
   // Poisson scratch (aliases ybuf storage; live only between the divergence
   // and the correction)
   double2 *spec;        // [k][kz][ky], k < nxm, ky <= nym/2
-  double *dstore;       // reciprocal Thomas pivots 1/d of the Poisson solve,
-                        // same indexing (tabulated by k_poisson_pivots)
+  double *dstore;       // reciprocal Thomas pivots of the Poisson solve [k][kz <= nzm/2][ky],
+                        // tabulated by k_poisson_pivots
   double *phi;          // pressure correction dph, [k][i][j], k < nxm
   // reference-boundary mode buffers (allocated on first use)
   double *qcap, *dq, *hro, *rhs;

@@ -630,41 +630,41 @@ __global__ void __launch_bounds__(FFT_T, 2) k_fft_z(BatchDev bt, int ns, FftSmem
 
 // ---------------------------------------------------------------------------
 // x: complex tridiagonal per mode (SolvePressureCorrection.F90:117-137),
-// marching k.  Row k of the normalised system is
-//   amph(k) x(k-1) + x(k) + apph(k) x(k+1) = dphc(k) s(k),
-//   s(k) = 1 / (acphk(k) - ak2(ky) - ak1(kz)).
-// dphc arrives unnormalised from the forward z transform and is scaled by
-// 1/(nym*nzm) here, before the scaling by s(k).  Its coefficients are real,
-// so the complex Thomas sweep is a real sweep applied to both parts.  The
-// (0,0) mode is singular (Neumann in x): its last equation is dropped and its
-// last unknown set to zero.
+// marching k.  Row k of mode (ky, kz) is
+//   amph(k) x(k-1) + (acphk(k) - ak2(ky) - ak1(kz)) x(k) + apph(k) x(k+1) = dphc(k),
+// with real coefficients, so the complex Thomas sweep (no pivoting: the rows
+// are diagonally dominant) is a real sweep applied to both parts.  dphc arrives
+// unnormalised from the forward z transform and is scaled by 1/(nym*nzm) here.
+// The (0,0) mode is singular (Neumann in x): its last equation is dropped and
+// its last unknown set to zero.
 //
 // The modified wavenumber is even, ak1(kz) = ak1(nzm - kz) bit for bit
 // (InitPressureSolver.F90:28-37 computes both from |kz|), so the modes kz and
-// nzm - kz of one ky have the same s(k) and the same pivots: one thread
-// solves both, the pivot table holds kz <= nzm/2 only, and the two chains
-// of the thread overlap each other's latency.
+// nzm - kz of one ky have the same pivots: the pivot table holds kz <= nzm/2
+// only, and k_poisson_x solves both in one thread, whose two chains overlap
+// each other's latency.
 // ---------------------------------------------------------------------------
 constexpr int KP_U = 4;   // planes per prefetch chunk of the sweeps
 
-// Row scale s(k) of mode (ak, ak1) and one step of the pivot recurrence
-// (zgttrf without pivoting): for row k >= 1 with am = amph(k) s(k),
-//   fact = am / d(k-1),  d(k) = 1 - fact * ap(k-1),  ap(k-1) = apph(k-1) s(k-1).
-// The sweep and the kernel that tabulates the pivots both go through these,
-// so the table holds the bits the sweep would compute.
-__device__ __forceinline__ double px_scale(const double *acph, int k, double ak, double ak1) {
-  return 1.0 / ((__ldg(acph + k) - ak) - ak1);
+// Reciprocal pivot of row k: r(k) = 1 / (acphk(k) - ak2 - ak1 - amph(k) apph(k-1) r(k-1)).
+__device__ __forceinline__ double px_pivot(double ac, double ak, double ak1, double am, double ap_prev, double r_prev) {
+  return 1.0 / __fma_rn(-(am * ap_prev), r_prev, (ac - ak) - ak1);
 }
-__device__ __forceinline__ double px_pivot(double am, double ap_prev, double &d) {
-  const double fact = am / d;
-  d = 1.0 - fact * ap_prev;
-  return fact;
+// Forward row y(k) = (f - amph(k) y(k-1)) r(k) and back row
+// x(k) = y(k) - apph(k) r(k) x(k+1), one multiply-add each on the serial chain.
+__device__ __forceinline__ double2 px_fwd(double2 f, double inv_norm, double am, double r, double2 y) {
+  const double c = am * r, g = inv_norm * r;
+  return make_double2(__fma_rn(-c, y.x, f.x * g), __fma_rn(-c, y.y, f.y * g));
+}
+__device__ __forceinline__ double2 px_bwd(double2 y, double ap, double r, double2 x) {
+  const double e = ap * r;
+  return make_double2(__fma_rn(-e, x.x, y.x), __fma_rn(-e, x.y, y.y));
 }
 
 // number of (kz <= nzm/2, ky) mode pairs of a box
 __host__ __device__ __forceinline__ long long px_pairs(int nzm, int nymh) { return (long long)(nzm / 2 + 1) * nymh; }
 
-// Reciprocal pivots 1/d(k) of the modes kz <= nzm/2 of one box, written to
+// Reciprocal pivots r(k) of the modes kz <= nzm/2 of one box, written to
 // B.dstore as [k][kz][ky].  They depend on the grid only, so a box computes
 // them once.
 __global__ void __launch_bounds__(256) k_poisson_pivots(BoxDev B) {
@@ -679,19 +679,18 @@ __global__ void __launch_bounds__(256) k_poisson_pivots(BoxDev B) {
   const double *acph = B.tab + (long long)T_ACPHK * B.nx;
   const double *apph = B.tab + (long long)T_APPHK * B.nx;
   double *__restrict__ dst = B.dstore + m;
-  double d = 1.0, ap_prev = 0.0;
+  double r = 0.0;
   for (int k = 0; k < nxm; ++k) {
-    const double s = px_scale(acph, k, ak, ak1);
-    if (k > 0) px_pivot(__ldg(amph + k) * s, ap_prev, d);
-    dst[(long long)k * np] = 1.0 / d;
-    ap_prev = __ldg(apph + k) * s;
+    r = px_pivot(__ldg(acph + k), ak, ak1, __ldg(amph + k), k ? __ldg(apph + k - 1) : 0.0, r);
+    dst[(long long)k * np] = r;
   }
 }
 
 // One thread per mode pair (kz, ky), (nzm - kz, ky) with kz <= nzm/2 (the
 // pair is a single mode for kz = 0 and kz = nzm/2), marching k: the forward
 // vector is written over the spectrum and read back by the back
-// substitution.
+// substitution.  The forward sweep recomputes the pivots (reading the table
+// there too would add 2 bytes per cell to the 36 that bound the kernel).
 __global__ void __launch_bounds__(256, 2) k_poisson_x(BatchDev bt, int ns) {
   const int b = find_box(bt.tile_off, bt.nbox, blockIdx.x);
   const BoxDev &B = bt.boxes[b];
@@ -711,11 +710,11 @@ __global__ void __launch_bounds__(256, 2) k_poisson_x(BatchDev bt, int ns) {
   const long long st = (long long)nzm * nh;                           // plane stride of the spectrum
   double2 *__restrict__ xa = B.spec + (long long)kz * nh + ky;        // mode kz
   double2 *__restrict__ xb = B.spec + (long long)(pair ? nzm - kz : kz) * nh + ky;   // mode nzm - kz
-  const double *__restrict__ rdt = B.dstore + m;                      // 1/d(k), by k_poisson_pivots
+  const double *__restrict__ rdt = B.dstore + m;                      // r(k), by k_poisson_pivots
   const bool zero_mode = (ky == 0 && kz == 0);
   const double inv_norm = 1.0 / ((double)B.nzm * (double)B.nym);     // the transforms' 1/(nym nzm)
-  // forward elimination (dgttrf + dgttrs forward sweep), planes in chunks
-  double d = 1.0, ap_prev = 0.0;
+  // forward elimination, planes in chunks
+  double r = 0.0, ap_prev = 0.0;
   double2 ya = make_double2(0.0, 0.0), yb = ya;
   for (int k0 = 0; k0 < nxm; k0 += KP_U) {
     double2 ra[KP_U], rb[KP_U];
@@ -729,32 +728,18 @@ __global__ void __launch_bounds__(256, 2) k_poisson_x(BatchDev bt, int ns) {
     for (int u = 0; u < KP_U; ++u) {
       const int k = k0 + u;
       if (k >= nxm) break;
-      const double s = px_scale(acph, k, ak, ak1);
-      double2 fa = ra[u], fb = rb[u];
-      fa.x = (fa.x * inv_norm) * s; fa.y = (fa.y * inv_norm) * s;
-      fb.x = (fb.x * inv_norm) * s; fb.y = (fb.y * inv_norm) * s;
-      if (k == 0) {
-        ya = fa;
-        yb = fb;
-      } else {
-        const double fact = px_pivot(__ldg(amph + k) * s, ap_prev, d);
-        ya.x = fa.x - fact * ya.x; ya.y = fa.y - fact * ya.y;
-        yb.x = fb.x - fact * yb.x; yb.y = fb.y - fact * yb.y;
-      }
+      const double am = __ldg(amph + k);
+      r = px_pivot(__ldg(acph + k), ak, ak1, am, ap_prev, r);
+      ya = px_fwd(ra[u], inv_norm, am, r, ya);
+      yb = px_fwd(rb[u], inv_norm, am, r, yb);
       xa[(long long)k * st] = ya;
       if (pair) xb[(long long)k * st] = yb;
-      ap_prev = __ldg(apph + k) * s;
+      ap_prev = __ldg(apph + k);
     }
   }
   // back substitution
-  double2 xna, xnb;
-  {
-    const double rd = rdt[(long long)(nxm - 1) * np];
-    xna = zero_mode ? make_double2(0.0, 0.0) : make_double2(ya.x * rd, ya.y * rd);
-    xnb = make_double2(yb.x * rd, yb.y * rd);
-  }
-  xa[(long long)(nxm - 1) * st] = xna;
-  if (pair) xb[(long long)(nxm - 1) * st] = xnb;
+  double2 xna = zero_mode ? make_double2(0.0, 0.0) : ya, xnb = yb;
+  if (zero_mode) xa[(long long)(nxm - 1) * st] = xna;
   for (int k0 = nxm - 2; k0 >= 0; k0 -= KP_U) {
     double2 yka[KP_U], ykb[KP_U];
     double rk[KP_U];
@@ -771,15 +756,97 @@ __global__ void __launch_bounds__(256, 2) k_poisson_x(BatchDev bt, int ns) {
     for (int u = 0; u < KP_U; ++u) {
       const int k = k0 - u;
       if (k < 0) break;
-      const double sk = px_scale(acph, k, ak, ak1);
-      const double ap = __ldg(apph + k) * sk;
-      xna.x = (yka[u].x - ap * xna.x) * rk[u];
-      xna.y = (yka[u].y - ap * xna.y) * rk[u];
-      xnb.x = (ykb[u].x - ap * xnb.x) * rk[u];
-      xnb.y = (ykb[u].y - ap * xnb.y) * rk[u];
+      const double ap = __ldg(apph + k);
+      xna = px_bwd(yka[u], ap, rk[u], xna);
+      xnb = px_bwd(ykb[u], ap, rk[u], xnb);
       xa[(long long)k * st] = xna;
       if (pair) xb[(long long)k * st] = xnb;
     }
+  }
+}
+
+// The x-solve of small sets, with the modes' columns on chip: one warp per 32
+// modes (a lane per mode, kz ky-contiguous), all rows copied into shared memory
+// at once, both sweeps there, pivots from the table KX_U rows ahead.  It moves
+// 20 bytes per cell and pays one load latency, where k_poisson_x pays one per
+// chunk of planes in either sweep: 49 us per launch on 65x64x64, 43 with the
+// reciprocal pivots of this form, 14 on chip.
+constexpr int KX_U = 8;
+__host__ __device__ constexpr int px_cols_bytes(int nxm) { return nxm * (32 * 16 + 16); }
+
+__global__ void __launch_bounds__(32) k_poisson_cols(BatchDev bt, int ns) {
+  extern __shared__ double2 psm[];
+  const int b = find_box(bt.tile_off, bt.nbox, blockIdx.x);
+  const BoxDev &B = bt.boxes[b];
+  if (!B.active || ns >= B.nsst) return;
+  if (B.sc->status != 0) return;
+  const int nh = B.nymh, nzm = B.nzm, nxm = B.nxm, lane = threadIdx.x;
+  const int st = nzm * nh;                       // modes, and plane stride of the spectrum
+  const int m = (blockIdx.x - __ldg(bt.tile_off + b)) * 32 + lane;
+  const bool ok = m < st;
+  const int mm = ok ? m : st - 1;                // lanes past the end repeat the last mode and store nothing
+  const int kz = mm / nh, ky = mm - kz * nh;
+  const long long np = px_pairs(nzm, nh);
+  double2 *__restrict__ const x = B.spec + mm;
+  const double *__restrict__ const rt = B.dstore + (long long)min(kz, nzm - kz) * nh + ky;
+  const double *amph = B.tab + (long long)T_AMPHK * B.nx, *apph = B.tab + (long long)T_APPHK * B.nx;
+  double2 *const s = psm + lane;                 // row k at s[32 k]
+  double2 *const t = psm + 32 * nxm;             // (amph, apph) of row k
+  for (int k = 0; k < nxm; ++k) cp_async16(s + 32 * k, x + (long long)k * st);
+  for (int k = lane; k < nxm; k += 32) {
+    cp_async8(&t[k].x, amph + k);
+    cp_async8(&t[k].y, apph + k);
+  }
+  cp_async_commit();
+  const double inv_norm = 1.0 / ((double)nzm * (double)B.nym);
+  double ra[KX_U];
+#pragma unroll
+  for (int u = 0; u < KX_U; ++u) ra[u] = rt[(long long)min(u, nxm - 1) * np];
+  cp_async_wait_all();
+  __syncwarp();
+  double2 y = make_double2(0.0, 0.0);
+  for (int k0 = 0; k0 < nxm; k0 += KX_U) {
+    double rn[KX_U];
+    double2 f[KX_U], a[KX_U];
+#pragma unroll
+    for (int u = 0; u < KX_U; ++u) {
+      rn[u] = rt[(long long)min(k0 + KX_U + u, nxm - 1) * np];
+      const int k = min(k0 + u, nxm - 1);
+      f[u] = s[32 * k];
+      a[u] = t[k];
+    }
+#pragma unroll
+    for (int u = 0; u < KX_U; ++u) {
+      if (k0 + u >= nxm) break;
+      y = px_fwd(f[u], inv_norm, a[u].x, ra[u], y);
+      s[32 * (k0 + u)] = y;
+    }
+#pragma unroll
+    for (int u = 0; u < KX_U; ++u) ra[u] = rn[u];
+  }
+  double2 xn = mm == 0 ? make_double2(0.0, 0.0) : y;
+  if (ok) x[(long long)(nxm - 1) * st] = xn;
+#pragma unroll
+  for (int u = 0; u < KX_U; ++u) ra[u] = rt[(long long)max(nxm - 2 - u, 0) * np];
+  for (int k0 = nxm - 2; k0 >= 0; k0 -= KX_U) {
+    double rn[KX_U];
+    double2 f[KX_U], a[KX_U];
+#pragma unroll
+    for (int u = 0; u < KX_U; ++u) {
+      rn[u] = rt[(long long)max(k0 - KX_U - u, 0) * np];
+      const int k = max(k0 - u, 0);
+      f[u] = s[32 * k];
+      a[u] = t[k];
+    }
+#pragma unroll
+    for (int u = 0; u < KX_U; ++u) {
+      const int k = k0 - u;
+      if (k < 0) break;
+      xn = px_bwd(f[u], a[u].y, ra[u], xn);
+      if (ok) x[(long long)k * st] = xn;
+    }
+#pragma unroll
+    for (int u = 0; u < KX_U; ++u) ra[u] = rn[u];
   }
 }
 

@@ -86,3 +86,32 @@ def test_on_chip_solves_match_oracle(ctx, nxm):
     err = compare_fields(box, s)
     assert all(v <= 1e-11 for v in err.values()), err
     ctx.remove_box(box)
+
+
+@pytest.mark.parametrize("nxm,nym,nzm", [(4, 8, 12), (9, 10, 9), (33, 60, 30), (436, 8, 12), (440, 8, 12)])
+def test_on_chip_pressure_solve_matches_oracle(ctx, nxm, nym, nzm):
+    """The x-solve with the modes' columns on chip (up to nxm = 438), over mode
+    counts that do not fill the last warp, and one box beyond it."""
+    cfg = cfg_of(nxm, nym, nzm, ylen=1.3, zlen=0.9, istr3=0 if nxm > 300 else 7)
+    s = oracle_state(cfg, seed=None)
+    s.dph[...] = np.random.default_rng(nxm).standard_normal(s.dph.shape)
+    box = ctx.add_box(cfg, s.g.xc, validate=False)
+    box.upload("dph", s.dph)
+    box.solve_pressure_correction()
+    O.solve_pressure_correction(s)
+    d, o = box.download("dph"), s.dph
+    assert np.linalg.norm((d - d.mean()) - (o - o.mean())) <= 1e-11 * np.linalg.norm(o - o.mean())
+    ctx.remove_box(box)
+
+
+def test_pressure_solve_forms_agree(ctx):
+    """The same bits on chip (one small box) and marched (in a large set)."""
+    cfg = cfg_of(40, 64, 30, dt=5e-4, ylen=1.3, zlen=0.9)
+    filler = [cfg_of(200, 320, 256, dt=1e-4)]     # two warps per SM: beyond four rounds
+    a, b = _boxes(ctx, [cfg])[0], _boxes(ctx, [cfg] + filler)
+    ctx.step([a], 2)
+    ctx.step(b, 2)
+    for f in FIELDS:
+        assert np.array_equal(a.download(f), b[0].download(f)), f
+    for x in [a] + b:
+        ctx.remove_box(x)
