@@ -367,7 +367,7 @@ struct FftSmem {
 // neighbouring blocks work on neighbouring tiles at the same time, the work
 // of boxes of different sizes spreads over all blocks, and a block changes
 // boxes at most once per run.  Runs are FFT_TILE_RUN long when every worker
-// of the grid (block, or warp of the warp transforms) gets at least that many
+// of the grid (block) gets at least that many
 // items, else 2 or 1 long, so that a small launch spreads over all workers.
 // A walker follows the tiles' boxes forward.
 constexpr int FFT_TILE_RUN = 4;
@@ -377,7 +377,8 @@ __device__ __forceinline__ int run_log2(int total, int workers) {
 struct TileRange {
   int t0, total, lgr;
   __device__ __forceinline__ explicit TileRange(int total_)
-      : total(total_), lgr(run_log2(total_, (int)gridDim.x)) { t0 = (int)blockIdx.x << lgr; }
+      : TileRange(total_, run_log2(total_, (int)gridDim.x)) {}
+  __device__ __forceinline__ TileRange(int total_, int lgr_) : total(total_), lgr(lgr_) { t0 = (int)blockIdx.x << lgr; }
   __device__ __forceinline__ int first() const { return t0 < total ? t0 : total; }
   __device__ __forceinline__ int next(int t) const {
     int n = t + 1;
@@ -646,10 +647,23 @@ __global__ void __launch_bounds__(FFT_T, 2) k_fft_z(BatchDev bt, int ns, FftSmem
 // ---------------------------------------------------------------------------
 constexpr int KP_U = 4;   // planes per prefetch chunk of the sweeps
 
-// Reciprocal pivot of row k: r(k) = 1 / (acphk(k) - ak2 - ak1 - amph(k) apph(k-1) r(k-1)).
-__device__ __forceinline__ double px_pivot(double ac, double ak, double ak1, double am, double ap_prev, double r_prev) {
-  return 1.0 / __fma_rn(-(am * ap_prev), r_prev, (ac - ak) - ak1);
-}
+// Reciprocal pivot r(k) of row k: the dgttrf recurrence without pivoting on
+// rows scaled to a unit diagonal, in LAPACK's operation order,
+//   s = 1 / (acphk - ak2 - ak1), fact = amph s / d(k-1), d(k) = 1 - fact apph(k-1) s(k-1),
+// and r = s / d.  The lowest modes lose digits in d to cancellation (their
+// columns are 1e-11 off at 384 planes); a pivot from sums of positive terms,
+// -(apph + t) with t(k) = lam + amph t(k-1) / (apph(k-1) + t(k-1)), is accurate to a
+// few roundings, but then differs from the reference's solver by that loss.
+struct PxPivot {
+  double d = 1.0, aps = 0.0;          // d(k-1), apph(k-1) s(k-1)
+  __device__ __forceinline__ double next(double am, double ac, double ap, double ak, double ak1) {
+    const double s = 1.0 / ((ac - ak) - ak1);
+    const double fact = am * s / d;   // amph(0) = 0
+    d = 1.0 - fact * aps;
+    aps = ap * s;
+    return s / d;
+  }
+};
 // Forward row y(k) = (f - amph(k) y(k-1)) r(k) and back row
 // x(k) = y(k) - apph(k) r(k) x(k+1), one multiply-add each on the serial chain.
 __device__ __forceinline__ double2 px_fwd(double2 f, double inv_norm, double am, double r, double2 y) {
@@ -679,11 +693,9 @@ __global__ void __launch_bounds__(256) k_poisson_pivots(BoxDev B) {
   const double *acph = B.tab + (long long)T_ACPHK * B.nx;
   const double *apph = B.tab + (long long)T_APPHK * B.nx;
   double *__restrict__ dst = B.dstore + m;
-  double r = 0.0;
-  for (int k = 0; k < nxm; ++k) {
-    r = px_pivot(__ldg(acph + k), ak, ak1, __ldg(amph + k), k ? __ldg(apph + k - 1) : 0.0, r);
-    dst[(long long)k * np] = r;
-  }
+  PxPivot piv;
+  for (int k = 0; k < nxm; ++k)
+    dst[(long long)k * np] = piv.next(__ldg(amph + k), __ldg(acph + k), __ldg(apph + k), ak, ak1);
 }
 
 // One thread per mode pair (kz, ky), (nzm - kz, ky) with kz <= nzm/2 (the
@@ -714,7 +726,7 @@ __global__ void __launch_bounds__(256, 2) k_poisson_x(BatchDev bt, int ns) {
   const bool zero_mode = (ky == 0 && kz == 0);
   const double inv_norm = 1.0 / ((double)B.nzm * (double)B.nym);     // the transforms' 1/(nym nzm)
   // forward elimination, planes in chunks
-  double r = 0.0, ap_prev = 0.0;
+  PxPivot piv;
   double2 ya = make_double2(0.0, 0.0), yb = ya;
   for (int k0 = 0; k0 < nxm; k0 += KP_U) {
     double2 ra[KP_U], rb[KP_U];
@@ -729,12 +741,11 @@ __global__ void __launch_bounds__(256, 2) k_poisson_x(BatchDev bt, int ns) {
       const int k = k0 + u;
       if (k >= nxm) break;
       const double am = __ldg(amph + k);
-      r = px_pivot(__ldg(acph + k), ak, ak1, am, ap_prev, r);
+      const double r = piv.next(am, __ldg(acph + k), __ldg(apph + k), ak, ak1);
       ya = px_fwd(ra[u], inv_norm, am, r, ya);
       yb = px_fwd(rb[u], inv_norm, am, r, yb);
       xa[(long long)k * st] = ya;
       if (pair) xb[(long long)k * st] = yb;
-      ap_prev = __ldg(apph + k);
     }
   }
   // back substitution
