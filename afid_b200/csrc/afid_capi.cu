@@ -7,14 +7,13 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <functional>
 #include <map>
 #include <string>
 #include <vector>
 
 #include "afid_device.cuh"
 #include "k_fft.cuh"
-#include "k_fftw.cuh"
+#include "k_fft2.cuh"
 #include "k_routine.cuh"
 #include "k_stencil.cuh"
 #include "../../include/afid_gpu.h"
@@ -50,13 +49,10 @@ int fail(int code, const char *fmt, ...) {
   } while (0)
 
 // Launch families; each has its own table of tile offsets per batch.  The
-// y transforms of boxes with a warp plan run in FAM_WY8/12 (values per
-// lane), the others in FAM_FY; likewise the z transforms in FAM_WZ8/12 and
-// FAM_FZ.
-enum Fam { FAM_K1 = 0, FAM_COL, FAM_CELL, FAM_DIAG, FAM_FY, FAM_FZ, FAM_PX, FAM_K2,
-           FAM_WY8, FAM_WY12, FAM_WZ8, FAM_WZ12, FAM_K1S, FAM_KS, FAM_PXS, NFAM };
-constexpr int WY_NV = 2;
-constexpr int WY_V[WY_NV] = {8, 12};
+// transforms of boxes with a two-pass plan run in FAM_Y2/FAM_Z2 + class, the
+// others in FAM_FY and FAM_FZ.
+enum Fam { FAM_K1 = 0, FAM_COL, FAM_CELL, FAM_DIAG, FAM_FY, FAM_FZ, FAM_PX, FAM_K2, FAM_K1S, FAM_KS, FAM_PXS,
+           FAM_Y2, FAM_Z2 = FAM_Y2 + 2, NFAM = FAM_Z2 + 2 };
 constexpr int HIST_CAP = 4096;
 
 struct HostBox {
@@ -73,6 +69,13 @@ struct HostBox {
   int nstatsamples = 0;
 };
 
+// shared memory (exchange buffer of ex_len values, then the twiddles) and
+// resident grid of a two-pass transform launch; [0, 1] y, [2, 3] z
+struct F2Shape {
+  size_t smem = 0;
+  int ex_len = 0, grid = 0;
+};
+
 struct Batch {
   std::vector<int> ids;
   BoxDev *d_boxes = nullptr;
@@ -86,9 +89,7 @@ struct Batch {
   size_t smem_ks = 0;               // shared memory of k_implicit_cols
   size_t smem_px = 0;               // shared memory of k_poisson_cols (0: the set runs k_poisson_x)
   int kseg = 0, nseg = 1;           // planes per block and blocks per column tile of the planewise marches
-  size_t smem_wy[WY_NV] = {};       // shared memory and resident grids of the warp y transforms
-  int grid_wy[WY_NV] = {};
-  int grid_wz[WY_NV] = {};          // resident grids of the warp z transforms (shared memory as y)
+  F2Shape f2[4];                    // two-pass transforms: y and z of classes 0 and 1
   cudaGraphExec_t gexec = nullptr;
   cudaStream_t gstream = nullptr;
   int graph_kernels = 0;    // kernel nodes of the captured step graph
@@ -129,57 +130,16 @@ int factor_radices(int n, int *rad, int *np) {
   return 0;
 }
 
-// Warp plan of an n-point transform (k_fftw.cuh): V values per lane (8 or
-// 12; 16 and 24 spilled registers at two blocks per SM), G = n / V lanes per
-// line (a power of two, min_g <= G <= 32), and a radix sequence whose
-// radices all divide V, power-of-two radices first; the fewest passes win,
-// then the fewer values per lane.  The y transforms need min_g = 2: their
-// staged rows (2 LPW rows of N + 2 doubles, or of N/2 + 1 complex values)
-// fit a warp buffer only with LPW = 32 / G <= 16.  Returns 0 (no plan) for
-// sizes the tile kernels keep: lines longer than WARP_PLAN_MAX_N, where the
-// tile kernels measured faster (384 and 768 points).
-constexpr int WARP_PLAN_MAX_N = WF_MAX_N;
-int warp_plan(int n, int *v_out, int *g_out, int *rad, int *np, int min_g = 1) {
-  static const int cand[7] = {16, 12, 8, 6, 4, 3, 2};
-  if (n > WARP_PLAN_MAX_N) return 0;
-  int best_v = 0, best_np = 99, best[8] = {};
-  for (int vi = 0; vi < WY_NV; ++vi) {
-    const int V = WY_V[vi];
-    if (n % V) continue;
-    const int G = n / V;
-    if (G < min_g || G > 32 || (G & (G - 1))) continue;
-    // depth-first search for the shortest factorisation into radices dividing V
-    int cur[8], found[8] = {}, found_np = 99;
-    std::function<void(int, int)> dfs = [&](int m, int d) {
-      if (d >= found_np || d >= 8) return;
-      if (m == 1) {
-        found_np = d;
-        for (int q = 0; q < d; ++q) found[q] = cur[q];
-        return;
-      }
-      for (int c : cand)
-        if (V % c == 0 && m % c == 0) {
-          cur[d] = c;
-          dfs(m / c, d + 1);
-        }
-    };
-    dfs(n, 0);
-    if (found_np < best_np) {
-      best_np = found_np;
-      best_v = V;
-      for (int q = 0; q < found_np; ++q) best[q] = found[q];
-    }
-  }
-  if (!best_v) return 0;
-  // power-of-two radices first (shift-and-mask indexing of the strides)
-  int o = 0;
-  for (int q = 0; q < best_np; ++q) if ((best[q] & (best[q] - 1)) == 0) rad[o++] = best[q];
-  for (int q = 0; q < best_np; ++q) if ((best[q] & (best[q] - 1)) != 0) rad[o++] = best[q];
-  *v_out = best_v;
-  *g_out = n / best_v;
-  *np = best_np;
-  return 1;
+// Two-pass plan of an n-point transform (k_fft2.cuh): n = r1 r2 with the
+// smallest larger radix r2; 0 where n has no two radices of the list.
+void two_pass_plan(int n, int *r) {
+  static const int rad[] = {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24, 25, 27, 30, 32};
+  r[0] = r[1] = 0;
+  for (int r2 : rad)
+    for (int r1 : rad)
+      if (!r[0] && r1 <= r2 && r1 * r2 == n) { r[0] = r1; r[1] = r2; }
 }
+int two_pass_class(const int *r) { return !r[0] ? -1 : r[1] > 16 ? 1 : 0; }
 
 // Variants of the explicit/forward kernel: tile height TI (block of 32 TI
 // threads), resident blocks per SM and planes per barrier.
@@ -202,12 +162,12 @@ long long tiles_of(const BoxDev &B, int fam, int k1_variant = 2, int k2_block = 
     case FAM_COL: return cdiv(B.plane, 256);
     case FAM_CELL: return cdiv((long long)B.nxm * B.plane, 256);
     case FAM_DIAG: return cdiv(B.plane, 256);
-    case FAM_FY: return B.wy_v ? 0 : (long long)B.nxm * cdiv(B.nzm, 2 * fft_y_pairs(B));
-    case FAM_WY8: case FAM_WY12:
-      return B.wy_v == WY_V[fam - FAM_WY8] ? (long long)B.nxm * wy_units_per_plane(B) : 0;
-    case FAM_FZ: return B.wz_v ? 0 : (long long)B.nxm * cdiv(B.nymh, fft_z_lines(B));
-    case FAM_WZ8: case FAM_WZ12:
-      return B.wz_v == WY_V[fam - FAM_WZ8] ? (long long)B.nxm * wz_units_per_plane(B) : 0;
+    case FAM_Y2: case FAM_Y2 + 1:
+      return two_pass_class(B.fy2) == fam - FAM_Y2 ? (long long)B.nxm * cdiv(B.nzm, 2 * f2_lines(B.fy2[0], B.fy2[1], false)) : 0;
+    case FAM_Z2: case FAM_Z2 + 1:
+      return two_pass_class(B.fz2) == fam - FAM_Z2 ? (long long)B.nxm * cdiv(B.nymh, f2_lines(B.fz2[0], B.fz2[1], true)) : 0;
+    case FAM_FY: return B.fy2[0] ? 0 : (long long)B.nxm * cdiv(B.nzm, 2 * fft_y_pairs(B));
+    case FAM_FZ: return B.fz2[0] ? 0 : (long long)B.nxm * cdiv(B.nymh, fft_z_lines(B));
     case FAM_PX: return cdiv(px_pairs(B.nzm, B.nymh), 256);
     case FAM_PXS: return cdiv((long long)B.nzm * B.nymh, 32);
   }
@@ -440,18 +400,18 @@ int get_box(afid_ctx *c, int id, HostBox **out) {
 }
 
 int init_kernel_attrs();
-int wy_shapes(const std::vector<BoxDev> &devs, const int *total, size_t *smem, int *grid, int *grid_z);
+int f2_shapes(const std::vector<BoxDev> &devs, const int *total, F2Shape *sh);
 
 
 // slot sizes (complex values) and twiddle lengths of the persistent
 // transforms, grown to cover box d (the directions d runs in a tile kernel)
 void fft_smem_grow(const BoxDev &d, FftSmem &y, FftSmem &z, int &twy, int &twz) {
-  if (!d.wy_v) {
+  if (!d.fy2[0]) {
     y.slot = std::max(y.slot, fft_y_slot(d.nym, fft_y_pairs(d)));
     y.tw = std::max(y.tw, d.nym);
     twy = std::max(twy, d.nym);
   }
-  if (!d.wz_v) {
+  if (!d.fz2[0]) {
     z.slot = std::max(z.slot, fft_z_lines(d) * d.nzm);
     z.tw = std::max(z.tw, d.nzm);
     twz = std::max(twz, d.nzm);
@@ -641,7 +601,7 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
     int rc = init_kernel_attrs();
     if (!rc) rc = fft_grid(k_fft_y_fwd, bt->smem_y, bt->total[FAM_FY], &bt->grid_y);
     if (!rc) rc = fft_grid(k_fft_z<-1>, bt->smem_z, bt->total[FAM_FZ], &bt->grid_z);
-    if (!rc) rc = wy_shapes(devs, bt->total, bt->smem_wy, bt->grid_wy, bt->grid_wz);
+    if (!rc) rc = f2_shapes(devs, bt->total, bt->f2);
     if (rc) { free_batch(bt); return rc; }
   }
   if (allow_split && n >= SPLIT_MIN_BOXES) {
@@ -670,72 +630,74 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
   return 0;
 }
 
-// Shared memory and resident grids (in blocks of wf_warps(V) warps, at
-// most one warp per unit) of the warp y and z transforms of a set of boxes.
-int wy_shapes(const std::vector<BoxDev> &devs, const int *total, size_t *smem, int *grid, int *grid_z) {
-  (void)devs;
+// Shared memory and resident grids of the two-pass transforms of a set of boxes.
+int f2_shapes(const std::vector<BoxDev> &devs, const int *total, F2Shape *sh) {
   int dev = 0, nsm = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  for (int c = 0; c < WY_NV; ++c) {
-    smem[c] = wf_smem_bytes(WY_V[c]);
-    grid[c] = grid_z[c] = 0;
-    for (int zd = 0; zd < 2; ++zd) {
-      const int units = total[(zd ? FAM_WZ8 : FAM_WY8) + c];
-      if (!units) continue;
-      int occ = 0;
-      const int nt = 32 * wf_warps(WY_V[c]);
-      if (c == 0 && !zd) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fftw_y_fwd<8>, nt, smem[c]));
-      else if (!zd) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fftw_y_fwd<12>, nt, smem[c]));
-      else if (c == 0) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fftw_z<-1, 8>, nt, smem[c]));
-      else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fftw_z<-1, 12>, nt, smem[c]));
-      if (occ < 1) return fail(AFID_ESIZE, "warp transform block of %zu bytes does not fit an SM", smem[c]);
-      (zd ? grid_z : grid)[c] = std::max(1, std::min((int)cdiv(units, wf_warps(WY_V[c])), nsm * occ));
+  for (int f = 0; f < 4; ++f) {
+    sh[f] = F2Shape{};
+    const int tiles = total[FAM_Y2 + f];
+    if (!tiles) continue;
+    int tw = 0;
+    for (const BoxDev &d : devs) {
+      const int *r = f < 2 ? d.fy2 : d.fz2;
+      if (two_pass_class(r) != (f & 1)) continue;
+      sh[f].ex_len = std::max(sh[f].ex_len, f2_exchange(r[0], r[1], f2_lines(r[0], r[1], f >= 2)));
+      tw = std::max(tw, r[0] * r[1]);
     }
+    sh[f].smem = (size_t)(sh[f].ex_len + tw) * 16;
+    int occ = 0;
+    if (f == 0) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fft2<F2_YF, -1, 0>, F2_T, sh[f].smem));
+    else if (f == 1) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fft2<F2_YF, -1, 1>, F2_T, sh[f].smem));
+    else if (f == 2) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fft2<F2_Z, -1, 0>, F2_T, sh[f].smem));
+    else CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_fft2<F2_Z, -1, 1>, F2_T, sh[f].smem));
+    if (occ < 1) return fail(AFID_ESIZE, "two-pass transform block of %zu bytes does not fit an SM", sh[f].smem);
+    sh[f].grid = std::max(1, std::min(tiles, nsm * occ));
   }
   return 0;
 }
 
 // The z transforms of a batch (SGN -1 forward, +1 inverse): the tile kernel
-// for boxes without a warp plan, one warp-kernel launch per class present.
+// for boxes without another plan, one launch per class of the other plans.
 template <int SGN, class BD>
-int launch_fft_z(const int *total, BD bd, int grid_z, size_t smem_z, FftSmem sm_z, const int *grid_wz,
-                 const size_t *smem_wy, cudaStream_t s, int ns) {
-  if (total[FAM_FZ] > 0) {
-    k_fft_z<SGN><<<grid_z, FFT_T, smem_z, s>>>(bd(FAM_FZ), ns, sm_z, total[FAM_FZ]);
+int launch_fft_z(const int *total, BD bd, int grid_z, size_t smem_z, FftSmem sm_z, const F2Shape *f2, cudaStream_t s, int ns) {
+  for (int c = 0; c < 2; ++c) {
+    const int f = FAM_Z2 + c;
+    const F2Shape &h = f2[2 + c];
+    if (!total[f]) continue;
+    if (c == 0) k_fft2<F2_Z, SGN, 0><<<h.grid, F2_T, h.smem, s>>>(bd(f), ns, h.ex_len, total[f]);
+    else k_fft2<F2_Z, SGN, 1><<<h.grid, F2_T, h.smem, s>>>(bd(f), ns, h.ex_len, total[f]);
     CKL();
   }
-  for (int c = 0; c < WY_NV; ++c) {
-    const int f = FAM_WZ8 + c;
-    if (!total[f]) continue;
-    if (c == 0) k_fftw_z<SGN, 8><<<grid_wz[c], 32 * wf_warps(8), smem_wy[c], s>>>(bd(f), ns, total[f]);
-    else k_fftw_z<SGN, 12><<<grid_wz[c], 32 * wf_warps(12), smem_wy[c], s>>>(bd(f), ns, total[f]);
+  if (total[FAM_FZ] > 0) {
+    k_fft_z<SGN><<<grid_z, FFT_T, smem_z, s>>>(bd(FAM_FZ), ns, sm_z, total[FAM_FZ]);
     CKL();
   }
   return 0;
 }
 
-// The y transforms of a batch: the tile kernel for boxes without a warp
-// plan, one warp-kernel launch per values-per-lane class present.
+// The y transforms of a batch: the tile kernel for boxes without another
+// plan, one launch per class of the other plans.
 template <class BD>
-int launch_fft_y(bool fwd, const int *total, BD bd, int grid_y, size_t smem_y, FftSmem sm_y, const int *grid_wy,
-                 const size_t *smem_wy, cudaStream_t s, int ns) {
-  if (total[FAM_FY] > 0) {
-    if (fwd) k_fft_y_fwd<<<grid_y, FFT_T, smem_y, s>>>(bd(FAM_FY), ns, sm_y, total[FAM_FY]);
-    else k_fft_y_inv<<<grid_y, FFT_T, smem_y, s>>>(bd(FAM_FY), ns, sm_y, total[FAM_FY]);
-    CKL();
-  }
-  for (int c = 0; c < WY_NV; ++c) {
-    const int f = FAM_WY8 + c;
+int launch_fft_y(bool fwd, const int *total, BD bd, int grid_y, size_t smem_y, FftSmem sm_y, const F2Shape *f2, cudaStream_t s, int ns) {
+  for (int c = 0; c < 2; ++c) {
+    const int f = FAM_Y2 + c;
+    const F2Shape &h = f2[c];
     if (!total[f]) continue;
     const BatchDev b = bd(f);
     if (c == 0) {
-      if (fwd) k_fftw_y_fwd<8><<<grid_wy[c], 32 * wf_warps(8), smem_wy[c], s>>>(b, ns, total[f]);
-      else k_fftw_y_inv<8><<<grid_wy[c], 32 * wf_warps(8), smem_wy[c], s>>>(b, ns, total[f]);
+      if (fwd) k_fft2<F2_YF, -1, 0><<<h.grid, F2_T, h.smem, s>>>(b, ns, h.ex_len, total[f]);
+      else k_fft2<F2_YI, +1, 0><<<h.grid, F2_T, h.smem, s>>>(b, ns, h.ex_len, total[f]);
     } else {
-      if (fwd) k_fftw_y_fwd<12><<<grid_wy[c], 32 * wf_warps(12), smem_wy[c], s>>>(b, ns, total[f]);
-      else k_fftw_y_inv<12><<<grid_wy[c], 32 * wf_warps(12), smem_wy[c], s>>>(b, ns, total[f]);
+      if (fwd) k_fft2<F2_YF, -1, 1><<<h.grid, F2_T, h.smem, s>>>(b, ns, h.ex_len, total[f]);
+      else k_fft2<F2_YI, +1, 1><<<h.grid, F2_T, h.smem, s>>>(b, ns, h.ex_len, total[f]);
     }
+    CKL();
+  }
+  if (total[FAM_FY] > 0) {
+    if (fwd) k_fft_y_fwd<<<grid_y, FFT_T, smem_y, s>>>(bd(FAM_FY), ns, sm_y, total[FAM_FY]);
+    else k_fft_y_inv<<<grid_y, FFT_T, smem_y, s>>>(bd(FAM_FY), ns, sm_y, total[FAM_FY]);
     CKL();
   }
   return 0;
@@ -775,14 +737,14 @@ int init_kernel_attrs() {
   CK(cudaFuncSetAttribute(k_fft_y_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
   CK(cudaFuncSetAttribute(k_fft_z<-1>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
   CK(cudaFuncSetAttribute(k_fft_z<+1>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
-  CK(cudaFuncSetAttribute(k_fftw_y_fwd<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
-  CK(cudaFuncSetAttribute(k_fftw_y_fwd<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
-  CK(cudaFuncSetAttribute(k_fftw_y_inv<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
-  CK(cudaFuncSetAttribute(k_fftw_y_inv<12>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
-  CK(cudaFuncSetAttribute(k_fftw_z<-1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
-  CK(cudaFuncSetAttribute(k_fftw_z<-1, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
-  CK(cudaFuncSetAttribute(k_fftw_z<+1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
-  CK(cudaFuncSetAttribute(k_fftw_z<+1, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+  CK(cudaFuncSetAttribute(k_fft2<F2_YF, -1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+  CK(cudaFuncSetAttribute(k_fft2<F2_YF, -1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+  CK(cudaFuncSetAttribute(k_fft2<F2_YI, +1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+  CK(cudaFuncSetAttribute(k_fft2<F2_YI, +1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+  CK(cudaFuncSetAttribute(k_fft2<F2_Z, -1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+  CK(cudaFuncSetAttribute(k_fft2<F2_Z, -1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+  CK(cudaFuncSetAttribute(k_fft2<F2_Z, +1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
+  CK(cudaFuncSetAttribute(k_fft2<F2_Z, +1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, fsm));
   done[dev] = true;
   return 0;
 }
@@ -854,13 +816,13 @@ int launch_poisson(const Batch *bt, cudaStream_t s, int ns, bool from_vel, Prof 
   }
   {
     int rc = launch_fft_y(true, bt->total, [&](int f) { return bdev(bt, f); }, bt->grid_y, bt->smem_y, bt->sm_y,
-                          bt->grid_wy, bt->smem_wy, s, ns);
+                          bt->f2, s, ns);
     if (rc) return rc;
   }
   PMARK(pf, AFID_K_FFT_Y_FWD);
   {
     int rc = launch_fft_z<-1>(bt->total, [&](int f) { return bdev(bt, f); }, bt->grid_z, bt->smem_z, bt->sm_z,
-                              bt->grid_wz, bt->smem_wy, s, ns);
+                              bt->f2, s, ns);
     if (rc) return rc;
   }
   PMARK(pf, AFID_K_FFT_Z_FWD);
@@ -871,13 +833,13 @@ int launch_poisson(const Batch *bt, cudaStream_t s, int ns, bool from_vel, Prof 
   PMARK(pf, AFID_K_POISSON_X);
   {
     int rc = launch_fft_z<+1>(bt->total, [&](int f) { return bdev(bt, f); }, bt->grid_z, bt->smem_z, bt->sm_z,
-                              bt->grid_wz, bt->smem_wy, s, ns);
+                              bt->f2, s, ns);
     if (rc) return rc;
   }
   PMARK(pf, AFID_K_FFT_Z_INV);
   {
     int rc = launch_fft_y(false, bt->total, [&](int f) { return bdev(bt, f); }, bt->grid_y, bt->smem_y, bt->sm_y,
-                          bt->grid_wy, bt->smem_wy, s, ns);
+                          bt->f2, s, ns);
     if (rc) return rc;
   }
   PMARK(pf, AFID_K_FFT_Y_INV);
@@ -1137,8 +1099,8 @@ int afid_box_add(afid_ctx *c, const afid_box_params *p, const double *xc, int *b
     delete hb;
     return fail(AFID_EFFT, "FFT size not efficient: nym=%d nzm=%d need prime factors <= 7 (code 444)", p->nym, p->nzm);
   }
-  if (!warp_plan(d.nym, &d.wy_v, &d.wy_g, d.wy_rad, &d.wy_np, 2)) d.wy_v = 0;
-  if (!warp_plan(d.nzm, &d.wz_v, &d.wz_g, d.wz_rad, &d.wz_np)) d.wz_v = 0;
+  two_pass_plan(d.nym, d.fy2);
+  two_pass_plan(d.nzm, d.fz2);
   Sizes s = sizes_of(*p);
   d.plane = s.plane; d.fsize = s.fsize; d.nspec = s.nspec;
   d.dx = (double)p->nxm / p->alx3; d.dy = (double)p->nym / p->ylen; d.dz = (double)p->nzm / p->zlen;
@@ -1591,9 +1553,10 @@ int afid_box_test_skip_z_copies(afid_ctx *c, int id, int skip, unsigned max_poll
   CK(cudaStreamSynchronize(c->stream));
   hb->dev.z_copy_skip = skip ? 1 : 0;
   hb->dev.mbar_tries = max_polls;
-  // the switch acts on the tile z kernel: a skipped box leaves the warp plan
+  // the switch acts on the tile z kernel: a skipped box leaves its two-pass plan
   BoxDev &d = hb->dev;
-  if (skip || !warp_plan(d.nzm, &d.wz_v, &d.wz_g, d.wz_rad, &d.wz_np)) d.wz_v = 0;
+  two_pass_plan(d.nzm, d.fz2);
+  if (skip) d.fz2[0] = 0;
   // batches hold copies of the descriptor: drop the ones with this box
   for (auto it = c->batches.begin(); it != c->batches.end();) {
     bool has = false;
@@ -2268,8 +2231,8 @@ extern "C" int afid_solve_pressure_correction_noalloc(double *dph, int nxm, int 
   memset(&d, 0, sizeof d);
   if (factor_radices(nym, d.fft_y_radix, &d.fft_y_np) || factor_radices(nzm, d.fft_z_radix, &d.fft_z_np))
     return fail(AFID_EFFT, "noalloc: nym=%d nzm=%d need prime factors <= 7", nym, nzm);
-  if (!warp_plan(nym, &d.wy_v, &d.wy_g, d.wy_rad, &d.wy_np, 2)) d.wy_v = 0;
-  if (!warp_plan(nzm, &d.wz_v, &d.wz_g, d.wz_rad, &d.wz_np)) d.wz_v = 0;
+  two_pass_plan(nym, d.fy2);
+  two_pass_plan(nzm, d.fz2);
   int dev = 0;
   CK(cudaGetDevice(&dev));
   int rc = noalloc_setup(dev);
@@ -2288,7 +2251,7 @@ extern "C" int afid_solve_pressure_correction_noalloc(double *dph, int nxm, int 
   const long long o_sc = (o_tw + 2LL * (nym + nzm) + 7) & ~7LL;
   const long long o_box = o_sc + (long long)((sizeof(BoxScalars) + 63) / 8);
   const long long o_off = o_box + (long long)((sizeof(BoxDev) + 63) / 8);
-  const long long o_tm = (o_off + 16 + 7) & ~7LL;   // 64-byte aligned TMA map of the z transform
+  const long long o_tm = (o_off + 32 + 7) & ~7LL;   // 64-byte aligned TMA map of the z transform
   if (o_tm + 16 > AFID_NOALLOC_DOUBLES) return fail(AFID_ESIZE, "noalloc: tables do not fit");
 
   // tables: the Poisson rows of InitPressureSolver.F90:22-59 (other k-tables unused)
@@ -2353,10 +2316,10 @@ extern "C" int afid_solve_pressure_correction_noalloc(double *dph, int nxm, int 
   // one-box tile tables of every family (only the transforms' and the
   // x-solve's are used)
   int off[NFAM][2], total[NFAM];
-  static_assert(sizeof(off) <= 16 * sizeof(double), "tile tables exceed their scratch slot");
+  static_assert(sizeof(off) <= 32 * sizeof(double), "tile tables exceed their scratch slot");
   for (int f = 0; f < NFAM; ++f) {
     off[f][0] = 0;
-    off[f][1] = total[f] = (f == FAM_FY || f == FAM_FZ || f == FAM_PX || f == FAM_PXS || (f >= FAM_WY8 && f <= FAM_WZ12)) ? (int)tiles_of(d, f) : 0;
+    off[f][1] = total[f] = (f == FAM_FY || f == FAM_FZ || f == FAM_PX || f == FAM_PXS || f >= FAM_Y2) ? (int)tiles_of(d, f) : 0;
   }
   CK(cudaMemcpyAsync(base + o_tab, tab, (size_t)n_tab * 8, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(base + o_tw, g_noalloc_host.tw, (size_t)(nym + nzm) * 16, cudaMemcpyHostToDevice, st));
@@ -2372,24 +2335,23 @@ extern "C" int afid_solve_pressure_correction_noalloc(double *dph, int nxm, int 
   fft_smem_grow(d, smy, smz, twy, twz);
   const size_t sy = (size_t)(2 * smy.slot + twy) * 16 + FFT_TAIL_BYTES;
   const size_t sz = (size_t)(2 * smz.slot + twz) * 16 + FFT_TAIL_BYTES;
-  size_t swy[WY_NV];
-  int gwy[WY_NV], gwz[WY_NV];
   rc = fft_grid(k_fft_y_fwd, sy, total[FAM_FY], &gy);
   if (!rc) rc = fft_grid(k_fft_z<-1>, sz, total[FAM_FZ], &gz);
-  if (!rc) rc = wy_shapes(std::vector<BoxDev>{d}, total, swy, gwy, gwz);
+  F2Shape f2[4];
+  if (!rc) rc = f2_shapes(std::vector<BoxDev>{d}, total, f2);
   if (rc) return rc;
   // the x-solve's pivots, for this call's grid
   k_poisson_pivots<<<(unsigned)cdiv(px_pairs(nzm, d.nymh), 256), 256, 0, st>>>(d);
   CKL();
-  rc = launch_fft_y(true, total, bd, gy, sy, smy, gwy, swy, st, 0);
+  rc = launch_fft_y(true, total, bd, gy, sy, smy, f2, st, 0);
   if (rc) return rc;
-  rc = launch_fft_z<-1>(total, bd, gz, sz, smz, gwz, swy, st, 0);
+  rc = launch_fft_z<-1>(total, bd, gz, sz, smz, f2, st, 0);
   if (rc) return rc;
   rc = launch_poisson_x(total, bd, px_cols_smem(nsm_of_device(), total[FAM_PXS], nxm, false), st, 0);
   if (rc) return rc;
-  rc = launch_fft_z<+1>(total, bd, gz, sz, smz, gwz, swy, st, 0);
+  rc = launch_fft_z<+1>(total, bd, gz, sz, smz, f2, st, 0);
   if (rc) return rc;
-  rc = launch_fft_y(false, total, bd, gy, sy, smy, gwy, swy, st, 0);
+  rc = launch_fft_y(false, total, bd, gy, sy, smy, f2, st, 0);
   if (rc) return rc;
   if (status) {
     // wait for this call's kernels and report its status word
