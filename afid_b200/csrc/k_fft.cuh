@@ -645,7 +645,7 @@ __global__ void __launch_bounds__(FFT_T, 2) k_fft_z(BatchDev bt, int ns, FftSmem
 // only, and k_poisson_x solves both in one thread, whose two chains overlap
 // each other's latency.
 // ---------------------------------------------------------------------------
-constexpr int KP_U = 4;   // planes per prefetch chunk of the sweeps
+constexpr int KP_U = 8;   // planes per chunk of k_poisson_x (ms per step at 192x384x384: 4 0.52, 6 0.75, 8 0.47)
 
 // Reciprocal pivot r(k) of row k: the dgttrf recurrence without pivoting on
 // rows scaled to a unit diagonal, in LAPACK's operation order,
@@ -699,10 +699,12 @@ __global__ void __launch_bounds__(256) k_poisson_pivots(BoxDev B) {
 }
 
 // One thread per mode pair (kz, ky), (nzm - kz, ky) with kz <= nzm/2 (the
-// pair is a single mode for kz = 0 and kz = nzm/2), marching k: the forward
-// vector is written over the spectrum and read back by the back
-// substitution.  The forward sweep recomputes the pivots (reading the table
-// there too would add 2 bytes per cell to the 36 that bound the kernel).
+// pair is a single mode for kz = 0 and kz = nzm/2), marching k in chunks of KP_U
+// planes.  The forward sweep keeps its vector in registers and stores one row
+// of it per chunk (the chunk's last, in place); the back substitution reads
+// the right-hand sides again, redoes a chunk's forward rows from the stored
+// one below, and writes the solution.  HBM traffic bounds the kernel: 29 bytes
+// per cell, where a forward vector written and read back took 36.
 __global__ void __launch_bounds__(256, 2) k_poisson_x(BatchDev bt, int ns) {
   const int b = find_box(bt.tile_off, bt.nbox, blockIdx.x);
   const BoxDev &B = bt.boxes[b];
@@ -714,62 +716,87 @@ __global__ void __launch_bounds__(256, 2) k_poisson_x(BatchDev bt, int ns) {
   if (m >= np) return;
   const int kz = (int)(m / nh), ky = (int)(m - (long long)kz * nh);
   const bool pair = kz > 0 && 2 * kz != nzm;
-  const double ak = __ldg(B.tab + (long long)T_NK * B.nx + nzm + ky);   // ak2(ky)
-  const double ak1 = __ldg(B.tab + (long long)T_NK * B.nx + kz);      // ak1(kz) = ak1(nzm - kz)
-  const double *amph = B.tab + (long long)T_AMPHK * B.nx;
-  const double *acph = B.tab + (long long)T_ACPHK * B.nx;
-  const double *apph = B.tab + (long long)T_APPHK * B.nx;
+  const double *__restrict__ amph = B.tab + (long long)T_AMPHK * B.nx;
+  const double *__restrict__ apph = B.tab + (long long)T_APPHK * B.nx;
   const long long st = (long long)nzm * nh;                           // plane stride of the spectrum
   double2 *__restrict__ xa = B.spec + (long long)kz * nh + ky;        // mode kz
   double2 *__restrict__ xb = B.spec + (long long)(pair ? nzm - kz : kz) * nh + ky;   // mode nzm - kz
   const double *__restrict__ rdt = B.dstore + m;                      // r(k), by k_poisson_pivots
   const bool zero_mode = (ky == 0 && kz == 0);
   const double inv_norm = 1.0 / ((double)B.nzm * (double)B.nym);     // the transforms' 1/(nym nzm)
-  // forward elimination, planes in chunks
-  PxPivot piv;
-  double2 ya = make_double2(0.0, 0.0), yb = ya;
-  for (int k0 = 0; k0 < nxm; k0 += KP_U) {
-    double2 ra[KP_U], rb[KP_U];
+  const int nch = (nxm + KP_U - 1) / KP_U;
+  double2 fa[KP_U], fb[KP_U];
+  double r[KP_U];
+  double2 ya = make_double2(0.0, 0.0), yb = ya;   // forward vector below the current chunk
+  for (int c = 0; c < nch - 1; ++c) {
+    const int k0 = c * KP_U;
 #pragma unroll
-    for (int u = 0; u < KP_U; ++u)
-      if (k0 + u < nxm) {
-        ra[u] = xa[(long long)(k0 + u) * st];
-        rb[u] = xb[(long long)(k0 + u) * st];   // = ra[u] for a single mode (not stored)
-      }
+    for (int u = 0; u < KP_U; ++u) {
+      fa[u] = xa[(long long)(k0 + u) * st];
+      fb[u] = xb[(long long)(k0 + u) * st];   // = fa[u] for a single mode (not stored)
+      r[u] = rdt[(long long)(k0 + u) * np];
+    }
+#pragma unroll
+    for (int u = 0; u < KP_U; ++u) {
+      const double am = __ldg(amph + k0 + u);
+      ya = px_fwd(fa[u], inv_norm, am, r[u], ya);
+      yb = px_fwd(fb[u], inv_norm, am, r[u], yb);
+    }
+    xa[(long long)(k0 + KP_U - 1) * st] = ya;
+    if (pair) xb[(long long)(k0 + KP_U - 1) * st] = yb;
+  }
+  double2 xna = make_double2(0.0, 0.0), xnb = xna, la = xna, lb = xna;   // x above, and the chunk's last forward row
+  for (int c = nch - 1; c >= 0; --c) {
+    const int k0 = c * KP_U;
+    const bool top = c == nch - 1;
 #pragma unroll
     for (int u = 0; u < KP_U; ++u) {
       const int k = k0 + u;
-      if (k >= nxm) break;
-      const double am = __ldg(amph + k);
-      const double r = piv.next(am, __ldg(acph + k), __ldg(apph + k), ak, ak1);
-      ya = px_fwd(ra[u], inv_norm, am, r, ya);
-      yb = px_fwd(rb[u], inv_norm, am, r, yb);
-      xa[(long long)k * st] = ya;
-      if (pair) xb[(long long)k * st] = yb;
+      if (k < nxm) {
+        if (top || u < KP_U - 1) {
+          fa[u] = xa[(long long)k * st];
+          fb[u] = xb[(long long)k * st];
+        }
+        r[u] = rdt[(long long)k * np];
+      }
     }
-  }
-  // back substitution
-  double2 xna = zero_mode ? make_double2(0.0, 0.0) : ya, xnb = yb;
-  if (zero_mode) xa[(long long)(nxm - 1) * st] = xna;
-  for (int k0 = nxm - 2; k0 >= 0; k0 -= KP_U) {
-    double2 yka[KP_U], ykb[KP_U];
-    double rk[KP_U];
+    if (!top) {
+      la = ya;
+      lb = yb;
+      if (c > 0) {
+        ya = xa[(long long)(k0 - 1) * st];
+        yb = xb[(long long)(k0 - 1) * st];
+      } else {
+        ya = yb = make_double2(0.0, 0.0);
+      }
+    }
+    double2 pa = ya, pb = yb;
 #pragma unroll
     for (int u = 0; u < KP_U; ++u) {
-      const int k = k0 - u;
-      if (k >= 0) {
-        yka[u] = xa[(long long)k * st];
-        ykb[u] = xb[(long long)k * st];
-        rk[u] = rdt[(long long)k * np];
+      if (k0 + u >= nxm) break;
+      if (top || u < KP_U - 1) {
+        const double am = __ldg(amph + k0 + u);
+        pa = px_fwd(fa[u], inv_norm, am, r[u], pa);
+        pb = px_fwd(fb[u], inv_norm, am, r[u], pb);
+        fa[u] = pa;
+        fb[u] = pb;
+      } else {
+        fa[u] = la;
+        fb[u] = lb;
       }
     }
 #pragma unroll
-    for (int u = 0; u < KP_U; ++u) {
-      const int k = k0 - u;
-      if (k < 0) break;
-      const double ap = __ldg(apph + k);
-      xna = px_bwd(yka[u], ap, rk[u], xna);
-      xnb = px_bwd(ykb[u], ap, rk[u], xnb);
+    for (int u = KP_U - 1; u >= 0; --u) {
+      const int k = k0 + u;
+      if (k >= nxm) continue;
+      if (k == nxm - 1) {
+        xna = zero_mode ? make_double2(0.0, 0.0) : fa[u];
+        xnb = fb[u];
+      } else {
+        const double ap = __ldg(apph + k);
+        xna = px_bwd(fa[u], ap, r[u], xna);
+        xnb = px_bwd(fb[u], ap, r[u], xnb);
+      }
       xa[(long long)k * st] = xna;
       if (pair) xb[(long long)k * st] = xnb;
     }
