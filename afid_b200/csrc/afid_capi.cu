@@ -67,6 +67,7 @@ struct HostBox {
   size_t out_doubles = 0;
   std::vector<double> stats;             // AFID_NSTAT x nxm accumulators (stat_arrays)
   int nstatsamples = 0;
+  int substep = 0;                       // the substep prepared last, whose coefficients the routines use
 };
 
 // shared memory (exchange buffer of ex_len values, then the twiddles) and
@@ -189,7 +190,7 @@ Sizes sizes_of(const afid_box_params &p) {
   s.scratch = pois > 4 * s.fsize ? pois : 4 * s.fsize;
   // tables + twiddles + coef + nu partials + history + scalars (in doubles)
   s.small = (long long)T_NK * s.nx + p.nzm + p.nym + 2LL * (p.nym + p.nzm) +
-            (long long)SYS_N * C_N * s.nx + 2 * NU_BLOCKS + (long long)HIST_CAP * HIST_FIELDS +
+            3LL * SYS_N * C_N * s.nx + 2 * NU_BLOCKS + (long long)HIST_CAP * HIST_FIELDS +
             (long long)(sizeof(BoxScalars) / 8 + 8) + s.plane +
             64;   // alignment of the scalars and the 128-byte TMA map (64-byte aligned)
   return s;
@@ -846,11 +847,8 @@ int launch_poisson(const Batch *bt, cudaStream_t s, int ns, bool from_vel, Prof 
   return 0;
 }
 
+// one prepared substep
 int launch_substep(const Batch *bt, cudaStream_t s, int ns, Prof *pf = nullptr) {
-  const int nb = (int)bt->ids.size();
-  k_substep_prep<<<nb, 256, 0, s>>>(bt->d_boxes, nb, ns);
-  CKL();
-  PMARK(pf, AFID_K_PREP);
   const BatchDev k1 = bdev(bt, FAM_K1);
   const int nk1 = bt->total[FAM_K1];
   if (nk1) switch (bt->k1_minb) {
@@ -884,19 +882,16 @@ int launch_step(const Batch *bt, cudaStream_t s, Prof *pf = nullptr) {
   launch_diag(bt, s, 0);
   CKL();
   PMARK(pf, AFID_K_DIAG);
-  k_finalize<<<cdiv(nb, 128), 128, 0, s>>>(bt->d_boxes, nb, 0);
+  k_substep_prep<<<dim3(nb, 3), 256, 0, s>>>(bt->d_boxes, nb, 0);
   CKL();
-  PMARK(pf, AFID_K_FINALIZE);
+  PMARK(pf, AFID_K_PREP);
   for (int ns = 0; ns < 3; ++ns) {
     int rc = launch_substep(bt, s, ns, pf);
     if (rc) return rc;
   }
-  k_plate_nu<<<dim3(NU_BLOCKS, nb), 256, 0, s>>>(bt->d_boxes, nb);
+  k_plate_nu<<<dim3(NU_BLOCKS, nb), 256, 0, s>>>(bt->d_boxes, nb, 1);
   CKL();
   PMARK(pf, AFID_K_PLATE_NU);
-  k_finalize<<<cdiv(nb, 128), 128, 0, s>>>(bt->d_boxes, nb, 1);
-  CKL();
-  PMARK(pf, AFID_K_FINALIZE);
   return 0;
 }
 
@@ -949,6 +944,14 @@ int ensure_routine_bufs(afid_ctx *c, HostBox *hb) {
     it = c->batches.erase(it);
   }
   return sync_self(hb);
+}
+
+// notes the substep the listed boxes are left at: ns, or the last of a step (-1)
+void note_substep(afid_ctx *c, const int *ids, int n, int ns) {
+  for (int b = 0; b < n; ++b) {
+    HostBox *hb = c->boxes[ids[b]];
+    if (ns < hb->prm.nsst) hb->substep = ns < 0 ? hb->prm.nsst - 1 : ns;
+  }
 }
 
 int single_batch(afid_ctx *c, int id, Batch **bt) { return get_batch(c, &id, 1, bt); }
@@ -1138,7 +1141,7 @@ int afid_box_add(afid_ctx *c, const afid_box_params *p, const double *xc, int *b
   o = (o + 1) & ~(size_t)1;
   d.twy = (const double2 *)(M + o); o += 2 * (size_t)p->nym;
   d.twz = (const double2 *)(M + o); o += 2 * (size_t)p->nzm;
-  d.coef = M + o; o += (size_t)SYS_N * C_N * d.nx;
+  d.coef = M + o; o += (size_t)3 * SYS_N * C_N * d.nx;
   d.nu_part = M + o; o += 2 * NU_BLOCKS;
   d.hist = M + o; o += (size_t)HIST_CAP * HIST_FIELDS;
   d.wall = M + o; o += (size_t)s.plane;
@@ -1643,6 +1646,7 @@ int afid_time_marcher_begin_substep(afid_ctx *c, int id, int ns) {
   if (rc) return rc;
   k_substep_prep<<<1, 256, 0, c->stream>>>(hb->d_self, 1, ns);
   CKL();
+  hb->substep = ns;
   return 0;
 }
 
@@ -1671,7 +1675,7 @@ static int implicit_one(afid_ctx *c, int id, int field) {
   rc = ensure_routine_bufs(c, hb);
   if (rc) return rc;
   const BoxDev &d = hb->dev;
-  k_implicit_one<<<(unsigned)cdiv(d.plane, 256), 256, 0, c->stream>>>(hb->d_self, field);
+  k_implicit_one<<<(unsigned)cdiv(d.plane, 256), 256, 0, c->stream>>>(hb->d_self, field, hb->substep);
   CKL();
   return 0;
 }
@@ -1692,7 +1696,7 @@ int afid_calc_local_divergence(afid_ctx *c, int id) {
   Batch *bt;
   rc = single_batch(c, id, &bt);
   if (rc) return rc;
-  launch_divergence(bt, c->stream, 0);
+  launch_divergence(bt, c->stream, c->boxes[id]->substep);
   CKL();
   return 0;
 }
@@ -1714,7 +1718,7 @@ static int correct(afid_ctx *c, int id, int vel, int pr) {
   Batch *bt;
   rc = single_batch(c, id, &bt);
   if (rc) return rc;
-  launch_correct(bt, c->stream, 0, vel, pr);
+  launch_correct(bt, c->stream, c->boxes[id]->substep, vel, pr);
   CKL();
   return 0;
 }
@@ -1770,7 +1774,7 @@ int afid_calc_plate_nu(afid_ctx *c, int id, double *nuslow, double *nusupp) {
   if (rc) return rc;
   rc = set_device(c);
   if (rc) return rc;
-  k_plate_nu<<<dim3(NU_BLOCKS, 1), 256, 0, c->stream>>>(hb->d_self, 1);
+  k_plate_nu<<<dim3(NU_BLOCKS, 1), 256, 0, c->stream>>>(hb->d_self, 1, 0);
   CKL();
   double part[2 * NU_BLOCKS];
   CK(cudaMemcpyAsync(part, hb->dev.nu_part, sizeof part, cudaMemcpyDeviceToHost, c->stream));
@@ -1791,6 +1795,9 @@ int afid_substep(afid_ctx *c, const int *ids, int n, int ns) {
   Batch *bt;
   rc = get_batch(c, ids, n, &bt);
   if (rc) return rc;
+  k_substep_prep<<<n, 256, 0, c->stream>>>(bt->d_boxes, n, ns);
+  CKL();
+  note_substep(c, ids, n, ns);
   return launch_substep(bt, c->stream, ns);
 }
 
@@ -1802,6 +1809,7 @@ int afid_step(afid_ctx *c, const int *ids, int n, int nsteps) {
   Batch *bt;
   rc = get_batch(c, ids, n, &bt);
   if (rc) return rc;
+  if (nsteps > 0) note_substep(c, ids, n, -1);
   for (int s = 0; s < nsteps; ++s) {
     rc = launch_step(bt, c->stream);
     if (rc) return rc;
@@ -1817,6 +1825,7 @@ int afid_step_profiled(afid_ctx *c, const int *ids, int n, int nsteps, double *k
   Batch *bt;
   rc = get_batch(c, ids, n, &bt);
   if (rc) return rc;
+  if (nsteps > 0) note_substep(c, ids, n, -1);
   for (int k = 0; k < nkernel; ++k) { kernel_ms[k] = 0.0; if (kernel_launches) kernel_launches[k] = 0; }
   for (int st = 0; st < nsteps; ++st) {
     Prof pf;
@@ -1903,6 +1912,7 @@ int afid_step_graph(afid_ctx *c, const int *ids, int n, int nsteps) {
   Batch *bt;
   rc = get_batch(c, ids, n, &bt);
   if (rc) return rc;
+  if (nsteps > 0) note_substep(c, ids, n, -1);
   if (bt->split && c->split_sets) {
     // each half steps on its own stream between a fork from and a join to
     // the context's stream; the halves are independent, so they need no

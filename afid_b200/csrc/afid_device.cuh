@@ -22,7 +22,8 @@ namespace afid {
 struct BoxScalars {
   double dt;        // current time step
   double time;      // simulation time
-  double al, ga, ro, beta;   // current substep coefficients, beta = dt/(2 Re)
+  // coefficients of the prepared substeps
+  struct Rk { double al, ga, ro, beta; } rk[3];   // beta = dt/(2 Re)
   double cfl;       // max CFL number of the current velocity (CalcMaxCFL)
   double cfl_used;  // cfl*dt (fixed dt) or cfl (variable dt), main.F90:171-189
   double divmax;    // max |div u| (CheckDivergence, without 1/(al dt))
@@ -44,6 +45,7 @@ struct BoxScalars {
   double tmax;
   int stop_ntime;
   int pad_hold_;
+  unsigned diag_blocks, nu_blocks;   // blocks of the box that have finished k_diag, k_plate_nu
 };
 
 // status of a box on hold: skipped like a failed box until resumed
@@ -57,10 +59,11 @@ enum TabId {
   T_G3RM, T_NK  // number of k-tables
 };
 
-// Per-substep tridiagonal tables in BoxDev::coef: for system s in
+// Per-substep tridiagonal tables in BoxDev::coef (one set of SYS_N * C_N * nx per
+// substep slot): for system s in
 // {SYS_X (vx, size nx), SYS_YZ (vy/vz, size nxm), SYS_T (temp, size nx)}
 // the arrays (sc, fact, dp, du, g, rd, ud) each of length nx at
-// coef[(s * C_N + a) * nx + k]; rd = 1/dp and ud = du/dp.
+// coef[((slot * SYS_N + s) * C_N + a) * nx + k]; rd = 1/dp and ud = du/dp.
 enum SysId { SYS_X = 0, SYS_YZ = 1, SYS_T = 2, SYS_N = 3 };
 enum CoefId { C_SC = 0, C_FACT, C_DP, C_DU, C_G, C_RD, C_UD, C_N };
 

@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(256) k_explicit_one(const BoxDev *__restrict__
 // and q += dq, with the wall rows of the size-nx systems taken from / left in
 // the carried rhs(1,:,:) plane exactly as the reference's shared rhs array
 // does.  Thread per (j, i) column.
-__global__ void __launch_bounds__(256) k_implicit_one(const BoxDev *__restrict__ boxes, int field) {
+__global__ void __launch_bounds__(256) k_implicit_one(const BoxDev *__restrict__ boxes, int field, int ns) {
   const BoxDev &B = boxes[0];
   const BoxScalars *S = B.sc;
   const long long P = B.plane;
@@ -68,11 +68,12 @@ __global__ void __launch_bounds__(256) k_implicit_one(const BoxDev *__restrict__
   const int i = (int)(col / B.nym);
   const int j = (int)(col - (long long)i * B.nym);
   const int nx = B.nx, nxm = B.nxm;
-  const double al = S->al, ga = S->ga, ro = S->ro, dt = S->dt;
+  const BoxScalars::Rk &rk = S->rk[ns];
+  const double al = rk.al, ga = rk.ga, ro = rk.ro, dt = S->dt;
   const double alre = al / B.ren, alpec = al / B.pec;
   const int sys = field == F_VX ? SYS_X : (field == F_T ? SYS_T : SYS_YZ);
-  const double *csc = coefp(B, sys, C_SC), *cf = coefp(B, sys, C_FACT);
-  const double *cdp = coefp(B, sys, C_DP), *cdu = coefp(B, sys, C_DU);
+  const double *csc = coefp(B, ns, sys, C_SC), *cf = coefp(B, ns, sys, C_FACT);
+  const double *cdp = coefp(B, ns, sys, C_DP), *cdu = coefp(B, ns, sys, C_DU);
   double *rhs = B.rhs;
   const int k0 = (field == F_VX || field == F_T) ? 1 : 0;
   const int n = (sys == SYS_YZ) ? nxm : nx;

@@ -136,8 +136,8 @@ __device__ __forceinline__ double bwd_row(double y, double rd, double ud, double
   return __fma_rn(-ud, x, y * rd);
 }
 
-__device__ __forceinline__ const double *coefp(const BoxDev &B, int sys, int arr) {
-  return B.coef + (long long)(sys * C_N + arr) * B.nx;
+__device__ __forceinline__ double *coefp(const BoxDev &B, int slot, int sys, int arr) {
+  return B.coef + (long long)((slot * SYS_N + sys) * C_N + arr) * B.nx;
 }
 
 // ---------------------------------------------------------------------------
@@ -146,9 +146,11 @@ __device__ __forceinline__ const double *coefp(const BoxDev &B, int sys, int arr
 // SolveImpEqnUpdate_YZ.F90:25-38, SolveImpEqnUpdate_Temp.F90:25-47), in the
 // dgttrf operation order without pivoting (the matrices are diagonally
 // dominant; a pivot that LAPACK would take is reported as status -2).
-// One block per box.
+// One block per box and substep: dt is fixed over a step, so a step prepares all
+// its substeps at once (blockIdx.y; a launch of one block per box prepares ns).
 // ---------------------------------------------------------------------------
 __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int ns) {
+  ns += blockIdx.y;
   const int b = blockIdx.x;
   if (b >= nbox) return;
   const BoxDev &B = boxes[b];
@@ -168,7 +170,7 @@ __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int n
     const double dt = S->dt;
     const double al = gam[ns] + rom[ns];
     const double beta = dt / B.ren * 0.5;     // TimeMarcher.F90:22
-    S->al = al; S->ga = gam[ns]; S->ro = rom[ns]; S->beta = beta;
+    S->rk[ns] = BoxScalars::Rk{al, gam[ns], rom[ns], beta};
     s_bx[SYS_X] = beta * al;
     s_bx[SYS_YZ] = beta * al;
     s_bx[SYS_T] = 0.5 * al * dt / B.pec;     // SolveImpEqnUpdate_Temp.F90:25
@@ -178,9 +180,7 @@ __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int n
   // row scale, sub- and super-diagonal (stored temporarily in C_FACT / C_DU)
   for (int t = threadIdx.x; t < 3 * nx; t += blockDim.x) {
     const int sys = t / nx, k = t % nx;
-    double *sc = B.coef + (long long)(sys * C_N + C_SC) * nx;
-    double *dl = B.coef + (long long)(sys * C_N + C_FACT) * nx;
-    double *du = B.coef + (long long)(sys * C_N + C_DU) * nx;
+    double *sc = coefp(B, ns, sys, C_SC), *dl = coefp(B, ns, sys, C_FACT), *du = coefp(B, ns, sys, C_DU);
     const double bx = s_bx[sys];
     double s = 1.0, am = 0.0, ap = 0.0;
     if (sys == SYS_X) {
@@ -209,10 +209,8 @@ __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int n
   if (threadIdx.x < 3) {
     const int sys = threadIdx.x;
     const int n = (sys == SYS_YZ) ? nxm : nx;
-    double *dl = B.coef + (long long)(sys * C_N + C_FACT) * nx;   // in: amkl, out: fact
-    double *du = B.coef + (long long)(sys * C_N + C_DU) * nx;
-    double *dp = B.coef + (long long)(sys * C_N + C_DP) * nx;
-    double *g = B.coef + (long long)(sys * C_N + C_G) * nx;
+    double *dl = coefp(B, ns, sys, C_FACT);   // in: amkl, out: fact
+    double *du = coefp(B, ns, sys, C_DU), *dp = coefp(B, ns, sys, C_DP), *g = coefp(B, ns, sys, C_G);
     double d = 1.0;
     dp[0] = 1.0;
     // rows k+1 of a chunk, read one chunk ahead: the chain of a row is then
@@ -254,7 +252,7 @@ __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int n
   __syncthreads();
   for (int t = threadIdx.x; t < 3 * nx; t += blockDim.x) {
     const int sys = t / nx, k = t % nx;
-    double *c = B.coef + (long long)(sys * C_N) * nx + k;
+    double *c = coefp(B, ns, sys, 0) + k;
     const double rd = 1.0 / c[(long long)C_DP * nx];
     c[(long long)C_RD * nx] = rd;
     c[(long long)C_UD * nx] = c[(long long)C_DU * nx] * rd;
@@ -307,7 +305,7 @@ struct RingAcc {
 };
 
 
-__device__ __forceinline__ const double *k1_tab_src(const BoxDev &B, int t, int k) {
+__device__ __forceinline__ const double *k1_tab_src(const BoxDev &B, int ns, int t, int k) {
   switch (t) {
     case KT_UDX3M: return B.tab + (long long)T_UDX3M * B.nx + k;
     case KT_UDX3C: return B.tab + (long long)T_UDX3C * B.nx + k;
@@ -317,12 +315,12 @@ __device__ __forceinline__ const double *k1_tab_src(const BoxDev &B, int t, int 
     case KT_AM3CK: return B.tab + (long long)T_AM3CK * B.nx + k;
     case KT_AC3CK: return B.tab + (long long)T_AC3CK * B.nx + k;
     case KT_AP3CK: return B.tab + (long long)T_AP3CK * B.nx + k;
-    case KT_XSC: return B.coef + (long long)(SYS_X * C_N + C_SC) * B.nx + k;
-    case KT_XF: return B.coef + (long long)(SYS_X * C_N + C_FACT) * B.nx + k;
-    case KT_YSC: return B.coef + (long long)(SYS_YZ * C_N + C_SC) * B.nx + k;
-    case KT_YF: return B.coef + (long long)(SYS_YZ * C_N + C_FACT) * B.nx + k;
-    case KT_TSC: return B.coef + (long long)(SYS_T * C_N + C_SC) * B.nx + k;
-    default: return B.coef + (long long)(SYS_T * C_N + C_FACT) * B.nx + k;
+    case KT_XSC: return coefp(B, ns, SYS_X, C_SC) + k;
+    case KT_XF: return coefp(B, ns, SYS_X, C_FACT) + k;
+    case KT_YSC: return coefp(B, ns, SYS_YZ, C_SC) + k;
+    case KT_YF: return coefp(B, ns, SYS_YZ, C_FACT) + k;
+    case KT_TSC: return coefp(B, ns, SYS_T, C_SC) + k;
+    default: return coefp(B, ns, SYS_T, C_FACT) + k;
   }
 }
 
@@ -392,7 +390,7 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
   const long long col = (long long)i * nym + j;
   const int nx = B.nx, nxm = B.nxm;
   const StencilConst c = make_sconst(B);
-  const double al = S->al, ga = S->ga, ro = S->ro, dt = S->dt;
+  const double al = S->rk[ns].al, ga = S->rk[ns].ga, ro = S->rk[ns].ro, dt = S->dt;
   const double alre = al / B.ren;
   const double alpec = al / B.pec;
   const double udy_al = B.dy * al;
@@ -412,7 +410,7 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
   // source of this thread's per-k scalar (threads tid < K1_NTAB), resolved
   // once: inside the march every descriptor read after a global store is a
   // reload, and the 14 cases would diverge within the first warp each plane
-  const double *tsrc = tid < K1_NTAB ? k1_tab_src(B, tid, 0) : nullptr;
+  const double *tsrc = tid < K1_NTAB ? k1_tab_src(B, ns, tid, 0) : nullptr;
   // the RK history of a plane travels with it in the ring: 4 fields x NT
   // columns as 2 NT aligned 16-byte pairs, two per thread.  Pair r = tid +
   // q NT is field r / (NT/2), tile row c / 16 and columns 2 (c % 16) + {0, 1}
@@ -572,7 +570,9 @@ __global__ void __launch_bounds__(256, 3) k_implicit_bwd(BatchDev bt, int ns) {
   // the LU rows of the three systems, as offsets from one base (seven
   // separate pointers would hold 14 registers across both sweeps)
   const double *__restrict__ cf = B.coef;
-  const auto lu = [&](int sys, int arr, int k) { return __ldg(cf + (long long)(sys * C_N + arr) * nx + k); };
+  const int set = ns * (SYS_N * C_N) * nx;      // the substep's set; int offsets: with 64-bit ones the loop spilled
+                                                // (64-box ensemble 1.33 ms per step, 1.24 so)
+  const auto lu = [&](int sys, int arr, int k) { return __ldg(cf + (set + (sys * C_N + arr) * nx + k)); };
   const double *__restrict__ y0 = B.ybuf[0] + col;
   const double *__restrict__ y1 = B.ybuf[1] + col;
   const double *__restrict__ y2 = B.ybuf[2] + col;
@@ -680,10 +680,10 @@ __global__ void __launch_bounds__(64) k_implicit_cols(BatchDev bt, int ns) {
   double *const rows = ksm + 8 * nxm + wp * nxm * KS_COLS;
   for (int k = lane; k < nxm; k += 32) {
     double *const t = reinterpret_cast<double *>(tab + 2 * k);
-    cp_async8(t, coefp(B, sys, C_FACT) + k);
-    cp_async8(t + 1, coefp(B, sys, C_G) + k);
-    cp_async8(t + 2, coefp(B, sys, C_RD) + k);
-    cp_async8(t + 3, coefp(B, sys, C_UD) + k);
+    cp_async8(t, coefp(B, ns, sys, C_FACT) + k);
+    cp_async8(t + 1, coefp(B, ns, sys, C_G) + k);
+    cp_async8(t + 2, coefp(B, ns, sys, C_RD) + k);
+    cp_async8(t + 3, coefp(B, ns, sys, C_UD) + k);
   }
   {
     const int p2 = 2 * (lane & 15);            // a pair of columns is inside the plane or outside (P is even)
@@ -792,10 +792,10 @@ __global__ void __launch_bounds__(256) k_correct(BatchDev bt, int ns, int do_vel
   double *__restrict__ vy = B.vy + col;
   double *__restrict__ vz = B.vz + col;
   double *__restrict__ pr = B.pr + col;
-  const double al = S->al, dt = S->dt;
+  const double al = S->rk[ns].al, dt = S->dt;
   const double udy = al * dt * B.dy;
   const double udz = al * dt * B.dz;
-  const double be = al * S->beta;
+  const double be = al * S->rk[ns].beta;
   const double dzq = B.dzq, dyq = B.dyq;
   const int ke = SEG ? min(ks + kseg, nxm) : nxm;
   double fm = phi[SEG ? (long long)max(ks - 1, 0) * P : 0];   // phi(kmv(k)): phi(0) for k = 0
@@ -882,7 +882,7 @@ __global__ void __launch_bounds__(256, 2) k_divergence(BatchDev bt, int ns, int 
   const double *__restrict__ vy = B.vy + col;
   const double *__restrict__ vz = B.vz + col;
   double *__restrict__ phi = B.phi + col;
-  const double usdtal = 1.0 / (S->dt * S->al);
+  const double usdtal = 1.0 / (S->dt * S->rk[ns].al);
   const double dz = B.dz, dy = B.dy;
   const double *__restrict__ t_udx3m = B.tab + (long long)T_UDX3M * B.nx;   // resolved before the stores
   const int ke = SEG ? min(ks + kseg, nxm) : nxm;
@@ -909,6 +909,86 @@ __global__ void __launch_bounds__(256, 2) k_divergence(BatchDev bt, int ns, int 
       xk = xn[u];
     }
   }
+}
+
+// Plate Nusselt numbers: blocks per box, fixed so that the order of the sum is.
+constexpr int NU_BLOCKS = 32;
+
+// Finalise the reductions of one box (one thread of the last of its blocks to
+// finish k_diag or k_plate_nu): diagnostics, plate Nu and the reference's error
+// codes.  What the other blocks wrote is read past L1.
+//   mode 0: step start  -> cfl/div/vmax from k_diag, then the dt rule of
+//           main.F90:171-189 (codes 165, 166)
+//   mode 1: step end    -> time += dt, ntime += 1, plate Nu, velocity limit
+//           (266, main.F90:204) and non-finite values (266)
+__device__ __forceinline__ void finalize_box(const BoxDev &B, int mode) {
+  BoxScalars *S = B.sc;
+  if (mode == 0) {
+    if (S->status != 0) return;
+    double cfl = __longlong_as_double((long long)__ldcg(&S->red_u64[0]));
+    S->divmax = __longlong_as_double((long long)__ldcg(&S->red_u64[1]));
+    S->vmax[1] = __longlong_as_double((long long)__ldcg(&S->red_u64[2]));
+    S->vmax[0] = __longlong_as_double((long long)__ldcg(&S->red_u64[3]));
+    for (int q = 0; q < 4; ++q) S->red_u64[q] = 0ull;
+    cfl = fmax(cfl, 0.00000001);             // CalcMaxCFL.F90:21
+    S->cfl = cfl;
+    if (__ldcg(&S->nonfinite)) { S->status = 266; return; }
+    // velocity limit (main.F90:204) and mass conservation (main.F90:220)
+    if (S->vmax[0] > S->limitvel && S->vmax[1] > S->limitvel) { S->status = 266; return; }
+    if (S->ntime >= 1 && S->resid > 0.0 && S->divmax > S->resid) { S->status = 169; return; }
+    double dt = S->dt;
+    if (S->idtv) {
+      if (S->ntime > 1) {
+        dt = (cfl < 1.0e-8) ? S->dtmax : S->cflmax / cfl;
+        if (dt > S->dtmax) dt = S->dtmax;
+      } else {
+        dt = S->dtmin;
+      }
+      S->dt = dt;
+      S->cfl_used = cfl;
+      if (dt < S->dtmin) S->status = 166;
+    } else {
+      S->cfl_used = cfl * dt;
+      if (S->cfl_used > S->cflmax) S->status = 165;
+    }
+  } else {
+    if (S->status != 0) return;
+    S->time += S->dt;
+    S->ntime += 1;
+    double lo = 0.0, up = 0.0;
+    for (int q = 0; q < NU_BLOCKS; ++q) { lo += __ldcg(B.nu_part + 2 * q); up += __ldcg(B.nu_part + 2 * q + 1); }
+    S->nu_bot = lo / (double)(B.nzm * B.nym);
+    S->nu_top = up / (double)(B.nzm * B.nym);
+    if (!isfinite(S->nu_bot) || !isfinite(S->nu_top)) S->status = 266;
+    if (B.hist_cap > 0) {
+      double *h = B.hist + (long long)((S->ntime - 1) % B.hist_cap) * HIST_FIELDS;
+      h[0] = S->time; h[1] = S->dt; h[2] = S->cfl_used; h[3] = S->divmax;
+      h[4] = S->nu_bot; h[5] = S->nu_top; h[6] = S->vmax[1]; h[7] = S->vmax[0];
+    }
+    // hold at the stop step or at an output time: main.F90's loop index is
+    // ntime - 1 here, so its "ntime.eq.1" is the second step
+    if (S->status == 0) {
+      bool hold = S->stop_ntime > 0 && S->ntime >= S->stop_ntime;
+      if (S->tout > 0.0 && (S->ntime == 2 || fmod(S->time, S->tout) < S->dt)) hold = true;
+      if (S->tmax > 0.0 && S->time > S->tmax) hold = true;
+      if (hold) S->status = AFID_STATUS_HELD_DEV;
+    }
+  }
+}
+
+// Whether the calling block is the last of n to arrive at *count (which the last
+// leaves at zero).  Every thread calls it; what the block wrote is visible to the
+// last block.
+__device__ __forceinline__ bool last_block(unsigned *count, unsigned n) {
+  __threadfence();
+  __syncthreads();
+  bool last = false;
+  if (threadIdx.x == 0) {
+    last = atomicAdd(count, 1u) == n - 1;
+    if (last) *count = 0;
+    __threadfence();
+  }
+  return __syncthreads_or(last);
 }
 
 // ---------------------------------------------------------------------------
@@ -990,12 +1070,16 @@ __global__ void __launch_bounds__(256, 2) k_diag(BatchDev bt, int every_box, int
     for (int q = 0; q < (int)(blockDim.x >> 5); ++q) m = fmax(m, sm[threadIdx.x][q]);
     atomicMax(&S->red_u64[threadIdx.x], dbits(m));
   }
+  if (!every_box) {
+    const unsigned segs = SEG ? (B.nxm + kseg - 1) / kseg : 1;
+    if (last_block(&S->diag_blocks, segs * (__ldg(bt.tile_off + b + 1) - __ldg(bt.tile_off + b))) && threadIdx.x == 0)
+      finalize_box(B, 0);
+  }
 }
 
 // Plate Nusselt numbers (CalcPlateNu.F90:24-43): per-block partial sums, in a
 // fixed number of blocks per box so that the final sum order is fixed.
-constexpr int NU_BLOCKS = 32;
-__global__ void __launch_bounds__(256) k_plate_nu(const BoxDev *__restrict__ boxes, int nbox) {
+__global__ void __launch_bounds__(256) k_plate_nu(const BoxDev *__restrict__ boxes, int nbox, int end_step) {
   const int b = blockIdx.y;
   if (b >= nbox) return;
   const BoxDev &B = boxes[b];
@@ -1017,6 +1101,7 @@ __global__ void __launch_bounds__(256) k_plate_nu(const BoxDev *__restrict__ box
     __syncthreads();
   }
   if (threadIdx.x == 0) { B.nu_part[2 * blockIdx.x] = s_lo[0]; B.nu_part[2 * blockIdx.x + 1] = s_up[0]; }
+  if (end_step && last_block(&B.sc->nu_blocks, NU_BLOCKS) && threadIdx.x == 0) finalize_box(B, 1);
 }
 
 // ---------------------------------------------------------------------------
@@ -1120,71 +1205,6 @@ __global__ void k_slab_gather(const BoxDev *__restrict__ bp, SlabList sl, int ns
     dst[P + c] = B.vy[o + c];
     dst[2 * P + c] = B.vz[o + c];
     dst[3 * P + c] = B.temp[o + c];
-  }
-}
-
-// Finalise the reductions of one box (thread per box): diagnostics, plate Nu
-// and the reference's error codes.
-//   mode 0: step start  -> cfl/div/vmax from k_diag, then the dt rule of
-//           main.F90:171-189 (codes 165, 166)
-//   mode 1: step end    -> time += dt, ntime += 1, plate Nu, velocity limit
-//           (266, main.F90:204) and non-finite values (266)
-__global__ void k_finalize(const BoxDev *__restrict__ boxes, int nbox, int mode) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nbox) return;
-  const BoxDev &B = boxes[b];
-  if (!B.active) return;
-  BoxScalars *S = B.sc;
-  if (mode == 0) {
-    if (S->status != 0) return;
-    double cfl = __longlong_as_double((long long)S->red_u64[0]);
-    S->divmax = __longlong_as_double((long long)S->red_u64[1]);
-    S->vmax[1] = __longlong_as_double((long long)S->red_u64[2]);
-    S->vmax[0] = __longlong_as_double((long long)S->red_u64[3]);
-    for (int q = 0; q < 4; ++q) S->red_u64[q] = 0ull;
-    cfl = fmax(cfl, 0.00000001);             // CalcMaxCFL.F90:21
-    S->cfl = cfl;
-    if (S->nonfinite) { S->status = 266; return; }
-    // velocity limit (main.F90:204) and mass conservation (main.F90:220)
-    if (S->vmax[0] > S->limitvel && S->vmax[1] > S->limitvel) { S->status = 266; return; }
-    if (S->ntime >= 1 && S->resid > 0.0 && S->divmax > S->resid) { S->status = 169; return; }
-    double dt = S->dt;
-    if (S->idtv) {
-      if (S->ntime > 1) {
-        dt = (cfl < 1.0e-8) ? S->dtmax : S->cflmax / cfl;
-        if (dt > S->dtmax) dt = S->dtmax;
-      } else {
-        dt = S->dtmin;
-      }
-      S->dt = dt;
-      S->cfl_used = cfl;
-      if (dt < S->dtmin) S->status = 166;
-    } else {
-      S->cfl_used = cfl * dt;
-      if (S->cfl_used > S->cflmax) S->status = 165;
-    }
-  } else {
-    if (S->status != 0) return;
-    S->time += S->dt;
-    S->ntime += 1;
-    double lo = 0.0, up = 0.0;
-    for (int q = 0; q < NU_BLOCKS; ++q) { lo += B.nu_part[2 * q]; up += B.nu_part[2 * q + 1]; }
-    S->nu_bot = lo / (double)(B.nzm * B.nym);
-    S->nu_top = up / (double)(B.nzm * B.nym);
-    if (!isfinite(S->nu_bot) || !isfinite(S->nu_top)) S->status = 266;
-    if (B.hist_cap > 0) {
-      double *h = B.hist + (long long)((S->ntime - 1) % B.hist_cap) * HIST_FIELDS;
-      h[0] = S->time; h[1] = S->dt; h[2] = S->cfl_used; h[3] = S->divmax;
-      h[4] = S->nu_bot; h[5] = S->nu_top; h[6] = S->vmax[1]; h[7] = S->vmax[0];
-    }
-    // hold at the stop step or at an output time: main.F90's loop index is
-    // ntime - 1 here, so its "ntime.eq.1" is the second step
-    if (S->status == 0) {
-      bool hold = S->stop_ntime > 0 && S->ntime >= S->stop_ntime;
-      if (S->tout > 0.0 && (S->ntime == 2 || fmod(S->time, S->tout) < S->dt)) hold = true;
-      if (S->tmax > 0.0 && S->time > S->tmax) hold = true;
-      if (hold) S->status = AFID_STATUS_HELD_DEV;
-    }
   }
 }
 

@@ -115,3 +115,34 @@ def test_pressure_solve_forms_agree(ctx):
         assert np.array_equal(a.download(f), b[0].download(f)), f
     for x in [a] + b:
         ctx.remove_box(x)
+
+
+@pytest.mark.parametrize("nsst,ns", [(3, 0), (3, 2), (1, 0)])
+def test_routines_use_the_substep_prepared_last(ctx, nsst, ns):
+    """A step prepares its substeps together; a routine called on its own uses
+    the substep begun last, whether that was by the routine-level call, by a
+    fused substep or (the last one) by a step."""
+    cfg = cfg_of(9, 10, 12, dt=1e-3, nsst=nsst)
+    s = oracle_state(cfg, seed=2)
+    s.vy[:9] = np.random.default_rng(1).standard_normal((9, 10, 12))
+    al = O.init_time_march_scheme(nsst)[2]
+    box = _boxes(ctx, [cfg])[0]
+
+    def div(a):
+        box.upload("vy", s.vy)
+        for f in ("vx", "vz"):
+            box.upload(f, np.zeros_like(s.vy))
+        box.calc_local_divergence()
+        t = O.State(**{**s.__dict__, "vx": np.zeros_like(s.vx), "vz": np.zeros_like(s.vz), "dph": s.dph.copy()})
+        O.calc_local_divergence(t, a, cfg.dt)
+        assert np.array_equal(box.download("dph"), t.dph)
+
+    ctx.step([box], 1)
+    div(al[nsst - 1])
+    box.time_marcher_begin_substep(ns)
+    div(al[ns])
+    ctx.substep([box], nsst - 1)
+    div(al[nsst - 1])
+    ctx.step([box], 1, graph=True)
+    div(al[nsst - 1])
+    ctx.remove_box(box)
