@@ -89,6 +89,7 @@ struct Batch {
   int k1s_seg = 0, k1s_nseg = 1;    // planes per block and blocks per tile of the K1 launch of the ks boxes
   size_t smem_ks = 0;               // shared memory of k_implicit_cols
   size_t smem_px = 0;               // shared memory of k_poisson_cols (0: the set runs k_poisson_x)
+  int nsst = 1;                     // most substeps of its boxes
   int kseg = 0, nseg = 1;           // planes per block and blocks per column tile of the planewise marches
   F2Shape f2[4];                    // two-pass transforms: y and z of classes 0 and 1
   cudaGraphExec_t gexec = nullptr;
@@ -587,6 +588,7 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
     off[(size_t)f * (n + 1) + n] = (int)acc;
     bt->total[f] = (int)acc;
   }
+  for (const BoxDev &d : devs) bt->nsst = std::max(bt->nsst, d.nsst);
   bt->smem_px = px_cols_smem(nsm, bt->total[FAM_PXS], devs[0].nxm, !allow_split);
   plane_segments(nsm, bt->total[FAM_COL], devs[0].nxm, &bt->kseg, &bt->nseg);
   k1s_segments(nsm, bt->total[FAM_K1S], devs[0].nxm, &bt->k1s_seg, &bt->k1s_nseg);
@@ -882,10 +884,10 @@ int launch_step(const Batch *bt, cudaStream_t s, Prof *pf = nullptr) {
   launch_diag(bt, s, 0);
   CKL();
   PMARK(pf, AFID_K_DIAG);
-  k_substep_prep<<<dim3(nb, 3), 256, 0, s>>>(bt->d_boxes, nb, 0);
+  k_substep_prep<<<dim3(nb, bt->nsst), 256, 0, s>>>(bt->d_boxes, nb, 0);
   CKL();
   PMARK(pf, AFID_K_PREP);
-  for (int ns = 0; ns < 3; ++ns) {
+  for (int ns = 0; ns < bt->nsst; ++ns) {   // a box of fewer substeps skips the others' launches
     int rc = launch_substep(bt, s, ns, pf);
     if (rc) return rc;
   }
