@@ -50,6 +50,8 @@ struct BoxScalars {
 
 // status of a box on hold: skipped like a failed box until resumed
 constexpr int AFID_STATUS_HELD_DEV = 1;
+// status of a box whose x-systems need a row exchange (k_substep_prep)
+constexpr int STATUS_PIVOT = -2;
 
 // Offsets of the metric tables inside BoxDev::tab (length nx each unless
 // noted).  Index k is 0-based (k = kc-1 of the reference).

@@ -145,9 +145,17 @@ __device__ __forceinline__ double *coefp(const BoxDev &B, int slot, int sys, int
 // the three x-tridiagonal matrices (SolveImpEqnUpdate_X.F90:25-44,
 // SolveImpEqnUpdate_YZ.F90:25-38, SolveImpEqnUpdate_Temp.F90:25-47), in the
 // dgttrf operation order without pivoting (the matrices are diagonally
-// dominant; a pivot that LAPACK would take is reported as status -2).
+// dominant; a row exchange that LAPACK would make is reported as STATUS_PIVOT).
 // One block per box and substep: dt is fixed over a step, so a step prepares all
 // its substeps at once (blockIdx.y; a launch of one block per box prepares ns).
+// The box then fails before any substep, as it does when they are prepared one
+// by one: writing a row's condition |d(k)| >= |amkl(k+1)| in e = 1/(beta al), its
+// margin grows with e, and the first substep has the largest al.
+//
+// Thread 0 decides for the block whether the box is skipped, since a block of
+// another substep may be writing -2 meanwhile.  A launch over all substeps
+// prepares them beside that one, so that what it leaves does not depend on
+// which block came first.
 // ---------------------------------------------------------------------------
 __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int ns) {
   ns += blockIdx.y;
@@ -156,8 +164,14 @@ __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int n
   const BoxDev &B = boxes[b];
   if (!B.active || ns >= B.nsst) return;
   BoxScalars *S = B.sc;
-  if (S->status != 0) return;
   __shared__ double s_bx[3];
+  __shared__ int s_skip;
+  if (threadIdx.x == 0) {
+    const int status = *(volatile int *)&S->status;
+    s_skip = status != 0 && !(gridDim.y > 1 && status == STATUS_PIVOT);
+  }
+  __syncthreads();
+  if (s_skip) return;
   if (threadIdx.x == 0) {
     double gam[3], rom[3];
     if (B.nsst > 1) {
@@ -247,7 +261,7 @@ __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int n
       for (int u = 0; u < U; ++u) { am[u] = amn[u]; up[u] = upn[u]; }
     }
     for (int k = n; k < nx; ++k) { dl[k] = 0.0; dp[k] = 1.0; g[k] = 0.0; }
-    if (pivot_needed) atomicExch(&S->status, -2);
+    if (pivot_needed) atomicExch(&S->status, STATUS_PIVOT);
   }
   __syncthreads();
   for (int t = threadIdx.x; t < 3 * nx; t += blockDim.x) {

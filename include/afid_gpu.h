@@ -23,6 +23,10 @@
  *     166 dt < dtmin, 169 divergence > resid, 266 velocity limit or a
  *     non-finite value; main.F90:184-220) and is skipped by later launches.
  *     Status 1 (AFID_STATUS_HELD) is a box on hold, not a failure.
+ *     Status -2 (no counterpart in the reference) marks a box whose x-systems
+ *     need a row exchange, which the LU without pivoting does not make (a dt
+ *     far beyond diffusion on a grid with a jump in spacing); the step that
+ *     finds it leaves the fields as they were.
  *     Status 990 (no counterpart in the reference) marks a box whose
  *     asynchronous tile copy did not complete within the kernel's wait
  *     limit; the kernel stops instead of waiting further.
