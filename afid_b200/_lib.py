@@ -41,7 +41,7 @@ EXPORTS = [
     "afid_global_quantities", "afid_calc_stats", "afid_calc_dissipation_nu", "afid_box_get_stats",
     "afid_box_reset_stats", "afid_slab_locations", "afid_slab_dump", "afid_box_set_time",
     "afid_box_interp_field", "afid_box_set_stop", "afid_box_resume",
-    "afid_box_test_skip_z_copies",
+    "afid_box_test_skip_z_copies", "afid_fft_tile_shape",
 ]
 
 STATS = ["vx_me", "vy_me", "vz_me", "temp_me", "vx_rms", "vy_rms", "vz_rms", "temp_rms", "tempvx_me",
@@ -78,6 +78,10 @@ class BoxScalars(C.Structure):
         ("divmax", C.c_double), ("vmax", C.c_double * 3), ("nu_bot", C.c_double),
         ("nu_top", C.c_double), ("ntime", C.c_int), ("status", C.c_int),
     ]
+
+
+class TileShape(C.Structure):
+    _fields_ = [(n, C.c_int) for n in ("y_tile", "z_tile", "y_pairs", "z_lines", "z_rows", "z_slot")]
 
 
 class StepRecord(C.Structure):
@@ -132,6 +136,7 @@ def lib(path: str | None = None) -> C.CDLL:
         "afid_step_profiled": ([vp, ip, i, i, dp, ip, i], i),
         "afid_solve_pressure_correction_noalloc": ([vp, i, i, i, dp, d, d, d, vp, ip], i),
         "afid_box_set_tuning": ([vp, i, i, i, i], i),
+        "afid_fft_tile_shape": ([i, i, i, i, C.POINTER(TileShape)], i),
         "afid_global_quantities": ([vp, i, C.POINTER(GlobalQ)], i),
         "afid_calc_stats": ([vp, i], i),
         "afid_calc_dissipation_nu": ([vp, i, dp, dp], i),

@@ -60,7 +60,7 @@ def fft_y_bytes(n: int, pairs: int) -> int:
 
 
 def fft_z_bytes(n: int, lines: int) -> int:
-    return (2 * lines * n + n) * 16 + TAIL_BYTES
+    return (2 * ((lines * n + 7) // 8 * 8) + n) * 16 + TAIL_BYTES
 
 
 def candidates(cfg: BouIn) -> dict:

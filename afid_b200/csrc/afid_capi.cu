@@ -320,11 +320,18 @@ EncodeTiledFn encode_tiled() {
   return fn;
 }
 
-// largest divisor of n not above 256 (kz rows per TMA box)
-int tma_rows(int n) {
-  for (int r = n < 256 ? n : 256; r > 1; --r)
-    if (n % r == 0) return r;
-  return 1;
+// kz rows per TMA box of a z tile of n rows of L values: the tile in one box, or
+// boxes whose ends keep the 128-byte alignment of the next one's destination
+// (r L a multiple of 8 values), with the fewest copies of boxes and, for the rest,
+// of single rows (fft_z_issue)
+int tma_rows(int n, int L) {
+  if (n <= 256) return n;
+  int best = 0, copies = 0;
+  for (int r = 256; r >= 1; --r) {
+    const int c = n / r + n % r;
+    if (r * L % 8 == 0 && (!best || c < copies)) { best = r; copies = c; }
+  }
+  return best;
 }
 
 // encode the z-transform map of box d (its spec array, box 2L x rb doubles)
@@ -332,7 +339,7 @@ int encode_z_map(BoxDev &d, CUtensorMap *out) {
   EncodeTiledFn fn = encode_tiled();
   if (!fn) return fail(AFID_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
   const int L = fft_z_lines(d);
-  d.fz_rb = tma_rows(d.nzm);
+  d.fz_rb = tma_rows(d.nzm, L);
   const cuuint64_t dims[2] = {(cuuint64_t)2 * d.nymh, (cuuint64_t)d.nxm * d.nzm};
   const cuuint64_t strides[1] = {(cuuint64_t)2 * d.nymh * sizeof(double)};
   const cuuint32_t box[2] = {(cuuint32_t)(2 * L), (cuuint32_t)d.fz_rb};
@@ -414,7 +421,7 @@ void fft_smem_grow(const BoxDev &d, FftSmem &y, FftSmem &z, int &twy, int &twz) 
     twy = std::max(twy, d.nym);
   }
   if (!d.fz2[0]) {
-    z.slot = std::max(z.slot, fft_z_lines(d) * d.nzm);
+    z.slot = std::max(z.slot, fft_z_slot(d.nzm, fft_z_lines(d)));
     z.tw = std::max(z.tw, d.nzm);
     twz = std::max(twz, d.nzm);
   }
@@ -1607,16 +1614,46 @@ int afid_box_history(afid_ctx *c, int id, afid_step_record *out, int max_records
   return n;
 }
 
+// lines per tile that the tile kernels take (0: the built-in choice)
+static int check_lines(int nym, int nzm, int fft_y_lines, int fft_z_lines) {
+  if (fft_y_lines < 0 || (fft_y_lines > 0 && !fft_y_ok(nym, fft_y_lines, FFT_SMEM_MAX)))
+    return fail(AFID_EINVAL, "fft_y_lines %d out of range", fft_y_lines);
+  if (fft_z_lines < 0 || (fft_z_lines > 0 && !fft_z_ok(nzm, fft_z_lines, FFT_SMEM_MAX)))
+    return fail(AFID_EINVAL, "fft_z_lines %d out of range", fft_z_lines);
+  return 0;
+}
+
+int afid_fft_tile_shape(int nym, int nzm, int y_lines, int z_lines, afid_tile_shape *out) {
+  if (!out) return fail(AFID_EINVAL, "null argument");
+  if (nym < 2 || nzm < 2 || nym % 2) return fail(AFID_EINVAL, "fft_tile_shape: need nzm >= 2 and an even nym >= 2");
+  if (nym > AFID_MAX_NYZ || nzm > AFID_MAX_NYZ) return fail(AFID_ESIZE, "fft_tile_shape: nym, nzm <= %d", AFID_MAX_NYZ);
+  BoxDev d{};
+  d.nym = nym; d.nzm = nzm; d.nymh = nym / 2 + 1;
+  if (factor_radices(nym, d.fft_y_radix, &d.fft_y_np) || factor_radices(nzm, d.fft_z_radix, &d.fft_z_np))
+    return fail(AFID_EFFT, "fft_tile_shape: nym=%d nzm=%d need prime factors <= 7", nym, nzm);
+  int rc = check_lines(nym, nzm, y_lines, z_lines);
+  if (rc) return rc;
+  two_pass_plan(nym, d.fy2);
+  two_pass_plan(nzm, d.fz2);
+  d.fy_lines = y_lines;
+  d.fz_lines = z_lines;
+  out->y_tile = d.fy2[0] == 0;
+  out->z_tile = d.fz2[0] == 0;
+  out->y_pairs = fft_y_pairs(d);
+  out->z_lines = fft_z_lines(d);
+  out->z_rows = tma_rows(nzm, out->z_lines);
+  out->z_slot = fft_z_slot(nzm, out->z_lines);
+  return 0;
+}
+
 int afid_box_set_tuning(afid_ctx *c, int id, int fft_y_lines, int fft_z_lines, int k1_minb) {
   if (!c) return fail(AFID_EINVAL, "null ctx");
   HostBox *hb;
   int rc = get_box(c, id, &hb);
   if (rc) return rc;
   BoxDev &d = hb->dev;
-  if (fft_y_lines < 0 || (fft_y_lines > 0 && !fft_y_ok(d.nym, fft_y_lines, FFT_SMEM_MAX)))
-    return fail(AFID_EINVAL, "fft_y_lines %d out of range", fft_y_lines);
-  if (fft_z_lines < 0 || (fft_z_lines > 0 && !fft_z_ok(d.nzm, fft_z_lines, FFT_SMEM_MAX)))
-    return fail(AFID_EINVAL, "fft_z_lines %d out of range", fft_z_lines);
+  rc = check_lines(d.nym, d.nzm, fft_y_lines, fft_z_lines);
+  if (rc) return rc;
   if (k1_minb != 0 && (k1_minb < K1_VMIN || k1_minb > K1_VMAX))
     return fail(AFID_EINVAL, "k1 variant must be 0 or %d..%d", K1_VMIN, K1_VMAX);
   rc = set_device(c);

@@ -113,7 +113,7 @@ struct BoxDev {
   int k1_minb;          // tuning: variant of the explicit/forward kernel (2, 3 or 4)
   int fy_lines;         // tuning: row pairs per y-FFT block (0 = default)
   int fz_lines;         // tuning: ky columns per z-FFT block (0 = default)
-  int fz_rb;            // kz rows per TMA box of the z transform (a divisor of nzm, <= 256)
+  int fz_rb;            // kz rows per TMA box of the z transform (<= 256, tma_rows)
   const CUtensorMap *tm_z;  // TMA map of spec as a 2-D FP64 array (2*nymh x nxm*nzm), box 2L x fz_rb
   int piv_ready;        // 1 = dstore holds the Poisson pivots of this grid
   // radices of the two-pass transforms (k_fft2.cuh), 0: the tile kernels run
@@ -231,7 +231,7 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, unsigned b
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
-// 2-D tile load of box (x, y) of ``map`` into shared memory at dst (16-byte
+// 2-D tile load of box (x, y) of ``map`` into shared memory at dst (128-byte
 // aligned); x times the element size must be a multiple of 16 bytes
 __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, unsigned long long *bar, int x,
                                             int y) {

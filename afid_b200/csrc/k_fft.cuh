@@ -318,6 +318,9 @@ constexpr int FFT_DEFAULT_LINES = 16;  // and the built-in choice at most
 // y: a slot holds the 2 Pp real rows of a forward tile (Pp N complex) or the
 // 2 Pp half-spectrum rows of an inverse tile (2 Pp (N/2+1) complex)
 __host__ __device__ __forceinline__ int fft_y_slot(int N, int Pp) { return 2 * Pp * (N / 2 + 1); }  // = Pp (N + 2)
+// z: a slot holds L lines, rounded up so that the second slot too starts on
+// the 128 bytes that the destination of a TMA copy needs
+__host__ __device__ __forceinline__ int fft_z_slot(int N, int L) { return (L * N + 7) & ~7; }
 // Dynamic shared memory of a transform block: two slots, the twiddles, then
 // the two slot mbarriers (16 bytes) and the cached box descriptor.  The
 // slots come first, at the start of the dynamic region, which keeps the TMA
@@ -326,7 +329,7 @@ constexpr int FFT_DESC_BYTES = (int)((sizeof(BoxDev) + 15) / 16 * 16);
 constexpr int FFT_TAIL_BYTES = 16 + FFT_DESC_BYTES;
 static_assert(FFT_TAIL_BYTES <= 1024, "the autotuner's size bound assumes a tail of at most 1 KB");
 __host__ __device__ __forceinline__ int fft_y_bytes(int N, int Pp) { return (2 * fft_y_slot(N, Pp) + N) * 16 + FFT_TAIL_BYTES; }
-__host__ __device__ __forceinline__ int fft_z_bytes(int N, int L) { return (2 * L * N + N) * 16 + FFT_TAIL_BYTES; }
+__host__ __device__ __forceinline__ int fft_z_bytes(int N, int L) { return (2 * fft_z_slot(N, L) + N) * 16 + FFT_TAIL_BYTES; }
 __host__ __device__ __forceinline__ bool fft_pow2(int v) { return v >= 1 && (v & (v - 1)) == 0; }
 __host__ __device__ __forceinline__ bool fft_y_ok(int N, int Pp, int budget) {
   return fft_pow2(Pp) && Pp <= FFT_MAX_LINES && Pp * N <= FFT_TILE_MAX && fft_y_bytes(N, Pp) <= budget;
@@ -551,17 +554,23 @@ struct ZDst {
 
 // The tile of L consecutive ky at all kz of plane k is a dense box of spec
 // seen as a 2-D FP64 array (2 nymh doubles per kz row, nxm nzm rows): one
-// thread loads it with nzm / fz_rb TMA copies of 2L x fz_rb doubles, which
-// land in shared memory as element (l, kz) at kz L + l; ky beyond nymh reads
-// as zero.  The copy of the next tile runs while the current one is
+// thread loads it with TMA copies of 2L x fz_rb doubles, which land in shared
+// memory as element (l, kz) at kz L + l; ky beyond nymh reads as zero.  A copy's
+// destination lies on 128 bytes: fz_rb L is a multiple of 8 values, or one copy
+// brings the whole tile (tma_rows).  The nzm mod fz_rb rows that are left come as
+// bulk copies of a row each (only the ky that exist: the other lines' values are
+// never stored).  The copy of the next tile runs while the current one is
 // transformed; each slot completes on its own mbarrier.
 __device__ __forceinline__ void fft_z_issue(const BoxDev &B, int lt, double2 *a, unsigned long long *bar) {
   const int N = B.nzm, nh = B.nymh, L = fft_z_lines(B), rb = B.fz_rb;
   const int ntl = (nh + L - 1) / L;
   const int k = lt / ntl, ky0 = (lt - k * ntl) * L;
-  mbar_expect_tx(bar, (unsigned)(16 * L * N));
+  const int whole = N / rb * rb, width = min(L, nh - ky0);
+  mbar_expect_tx(bar, (unsigned)(16 * (L * whole + width * (N - whole))));
   if (B.z_copy_skip) return;   // test switch: the wait on this slot runs out
-  for (int c = 0; c < N / rb; ++c) tma_load_2d(a + c * rb * L, B.tm_z, bar, 2 * ky0, k * N + c * rb);
+  for (int r = 0; r < whole; r += rb) tma_load_2d(a + r * L, B.tm_z, bar, 2 * ky0, k * N + r);
+  const double2 *const row = B.spec + (long long)k * N * nh + ky0;
+  for (int r = whole; r < N; ++r) bulk_load(a + r * L, row + (long long)r * nh, (unsigned)(16 * width), bar);
 }
 
 template <int SGN>

@@ -211,6 +211,15 @@ int afid_box_test_skip_z_copies(afid_ctx *ctx, int box_id, int skip, unsigned ma
  * four, five or six blocks; 6 = 32x2 tiles, eight blocks (0 = 4).  Results
  * do not depend on these values. */
 int afid_box_set_tuning(afid_ctx *ctx, int box_id, int fft_y_lines, int fft_z_lines, int k1_minb);
+/* Transform tiles of nym x nzm lines with the given lines per tile (as
+ * afid_box_set_tuning takes them; host only, no counterpart in the reference). */
+typedef struct afid_tile_shape {
+  int y_tile, z_tile;   /* 1: the lines run in the tile kernels, 0: in two register passes */
+  int y_pairs;          /* row pairs of a y tile */
+  int z_lines, z_rows;  /* ky of a z tile, kz rows of one of its tile copies */
+  int z_slot;           /* complex values from one z slot in shared memory to the next */
+} afid_tile_shape;
+int afid_fft_tile_shape(int nym, int nzm, int fft_y_lines, int fft_z_lines, afid_tile_shape *out);
 /* Copies up to max_records of the most recent per-step records, oldest
  * first; returns the number copied (>= 0) or an error code. */
 int afid_box_history(afid_ctx *ctx, int box_id, afid_step_record *out, int max_records);
