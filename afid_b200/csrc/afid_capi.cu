@@ -67,7 +67,6 @@ struct HostBox {
   size_t out_doubles = 0;
   std::vector<double> stats;             // AFID_NSTAT x nxm accumulators (stat_arrays)
   int nstatsamples = 0;
-  int substep = 0;                       // the substep prepared last, whose coefficients the routines use
 };
 
 // shared memory (exchange buffer of ex_len values, then the twiddles) and
@@ -955,14 +954,6 @@ int ensure_routine_bufs(afid_ctx *c, HostBox *hb) {
   return sync_self(hb);
 }
 
-// notes the substep the listed boxes are left at: ns, or the last of a step (-1)
-void note_substep(afid_ctx *c, const int *ids, int n, int ns) {
-  for (int b = 0; b < n; ++b) {
-    HostBox *hb = c->boxes[ids[b]];
-    if (ns < hb->prm.nsst) hb->substep = ns < 0 ? hb->prm.nsst - 1 : ns;
-  }
-}
-
 int single_batch(afid_ctx *c, int id, Batch **bt) { return get_batch(c, &id, 1, bt); }
 
 }  // namespace
@@ -1685,7 +1676,6 @@ int afid_time_marcher_begin_substep(afid_ctx *c, int id, int ns) {
   if (rc) return rc;
   k_substep_prep<<<1, 256, 0, c->stream>>>(hb->d_self, 1, ns);
   CKL();
-  hb->substep = ns;
   return 0;
 }
 
@@ -1714,7 +1704,7 @@ static int implicit_one(afid_ctx *c, int id, int field) {
   rc = ensure_routine_bufs(c, hb);
   if (rc) return rc;
   const BoxDev &d = hb->dev;
-  k_implicit_one<<<(unsigned)cdiv(d.plane, 256), 256, 0, c->stream>>>(hb->d_self, field, hb->substep);
+  k_implicit_one<<<(unsigned)cdiv(d.plane, 256), 256, 0, c->stream>>>(hb->d_self, field);
   CKL();
   return 0;
 }
@@ -1735,7 +1725,7 @@ int afid_calc_local_divergence(afid_ctx *c, int id) {
   Batch *bt;
   rc = single_batch(c, id, &bt);
   if (rc) return rc;
-  launch_divergence(bt, c->stream, c->boxes[id]->substep);
+  launch_divergence(bt, c->stream, -1);   // the substep prepared last
   CKL();
   return 0;
 }
@@ -1757,7 +1747,7 @@ static int correct(afid_ctx *c, int id, int vel, int pr) {
   Batch *bt;
   rc = single_batch(c, id, &bt);
   if (rc) return rc;
-  launch_correct(bt, c->stream, c->boxes[id]->substep, vel, pr);
+  launch_correct(bt, c->stream, -1, vel, pr);   // the substep prepared last
   CKL();
   return 0;
 }
@@ -1836,7 +1826,6 @@ int afid_substep(afid_ctx *c, const int *ids, int n, int ns) {
   if (rc) return rc;
   k_substep_prep<<<n, 256, 0, c->stream>>>(bt->d_boxes, n, ns);
   CKL();
-  note_substep(c, ids, n, ns);
   return launch_substep(bt, c->stream, ns);
 }
 
@@ -1848,7 +1837,6 @@ int afid_step(afid_ctx *c, const int *ids, int n, int nsteps) {
   Batch *bt;
   rc = get_batch(c, ids, n, &bt);
   if (rc) return rc;
-  if (nsteps > 0) note_substep(c, ids, n, -1);
   for (int s = 0; s < nsteps; ++s) {
     rc = launch_step(bt, c->stream);
     if (rc) return rc;
@@ -1864,7 +1852,6 @@ int afid_step_profiled(afid_ctx *c, const int *ids, int n, int nsteps, double *k
   Batch *bt;
   rc = get_batch(c, ids, n, &bt);
   if (rc) return rc;
-  if (nsteps > 0) note_substep(c, ids, n, -1);
   for (int k = 0; k < nkernel; ++k) { kernel_ms[k] = 0.0; if (kernel_launches) kernel_launches[k] = 0; }
   for (int st = 0; st < nsteps; ++st) {
     Prof pf;
@@ -1951,7 +1938,6 @@ int afid_step_graph(afid_ctx *c, const int *ids, int n, int nsteps) {
   Batch *bt;
   rc = get_batch(c, ids, n, &bt);
   if (rc) return rc;
-  if (nsteps > 0) note_substep(c, ids, n, -1);
   if (bt->split && c->split_sets) {
     // each half steps on its own stream between a fork from and a join to
     // the context's stream; the halves are independent, so they need no

@@ -22,8 +22,9 @@ namespace afid {
 struct BoxScalars {
   double dt;        // current time step
   double time;      // simulation time
-  // coefficients of the prepared substeps
-  struct Rk { double al, ga, ro, beta; } rk[3];   // beta = dt/(2 Re)
+  // coefficients of the substep prepared last, which the routine-level calls
+  // use, then of the prepared substeps: rk[1 + ns], and rk[0] for ns = -1
+  struct Rk { double al, ga, ro, beta; } rk[4];   // beta = dt/(2 Re)
   double cfl;       // max CFL number of the current velocity (CalcMaxCFL)
   double cfl_used;  // cfl*dt (fixed dt) or cfl (variable dt), main.F90:171-189
   double divmax;    // max |div u| (CheckDivergence, without 1/(al dt))
@@ -45,6 +46,8 @@ struct BoxScalars {
   double tmax;
   int stop_ntime;
   int pad_hold_;
+  int cur;          // the substep prepared last (rk[0]), whose tables the routines use
+  int pad_cur_;
   unsigned diag_blocks, nu_blocks;   // blocks of the box that have finished k_diag, k_plate_nu
 };
 

@@ -58,8 +58,8 @@ __global__ void __launch_bounds__(256) k_explicit_one(const BoxDev *__restrict__
 // history update, forward elimination into the rhs buffer, back substitution
 // and q += dq, with the wall rows of the size-nx systems taken from / left in
 // the carried rhs(1,:,:) plane exactly as the reference's shared rhs array
-// does.  Thread per (j, i) column.
-__global__ void __launch_bounds__(256) k_implicit_one(const BoxDev *__restrict__ boxes, int field, int ns) {
+// does.  Thread per (j, i) column, with the substep prepared last.
+__global__ void __launch_bounds__(256) k_implicit_one(const BoxDev *__restrict__ boxes, int field) {
   const BoxDev &B = boxes[0];
   const BoxScalars *S = B.sc;
   const long long P = B.plane;
@@ -68,7 +68,8 @@ __global__ void __launch_bounds__(256) k_implicit_one(const BoxDev *__restrict__
   const int i = (int)(col / B.nym);
   const int j = (int)(col - (long long)i * B.nym);
   const int nx = B.nx, nxm = B.nxm;
-  const BoxScalars::Rk &rk = S->rk[ns];
+  const int ns = S->cur;
+  const BoxScalars::Rk &rk = S->rk[0];
   const double al = rk.al, ga = rk.ga, ro = rk.ro, dt = S->dt;
   const double alre = al / B.ren, alpec = al / B.pec;
   const int sys = field == F_VX ? SYS_X : (field == F_T ? SYS_T : SYS_YZ);

@@ -168,28 +168,31 @@ __global__ void k_substep_prep(const BoxDev *__restrict__ boxes, int nbox, int n
   __shared__ int s_skip;
   if (threadIdx.x == 0) {
     const int status = *(volatile int *)&S->status;
+    const double dt = S->dt;
     s_skip = status != 0 && !(gridDim.y > 1 && status == STATUS_PIVOT);
+    if (!s_skip) {
+      double gam[3], rom[3];
+      if (B.nsst > 1) {
+        gam[0] = 8.0 / 15.0; gam[1] = 5.0 / 12.0; gam[2] = 3.0 / 4.0;
+        rom[0] = 0.0; rom[1] = -17.0 / 60.0; rom[2] = -5.0 / 12.0;
+      } else {
+        gam[0] = 1.5; gam[1] = 0.0; gam[2] = 0.0;
+        rom[0] = -0.5; rom[1] = 0.0; rom[2] = 0.0;
+      }
+      const double al = gam[ns] + rom[ns];
+      const double beta = dt / B.ren * 0.5;     // TimeMarcher.F90:22
+      S->rk[1 + ns] = BoxScalars::Rk{al, gam[ns], rom[ns], beta};
+      if (gridDim.y == 1 || ns == B.nsst - 1) {
+        S->rk[0] = BoxScalars::Rk{al, gam[ns], rom[ns], beta};
+        S->cur = ns;
+      }
+      s_bx[SYS_X] = beta * al;
+      s_bx[SYS_YZ] = beta * al;
+      s_bx[SYS_T] = 0.5 * al * dt / B.pec;     // SolveImpEqnUpdate_Temp.F90:25
+    }
   }
   __syncthreads();
   if (s_skip) return;
-  if (threadIdx.x == 0) {
-    double gam[3], rom[3];
-    if (B.nsst > 1) {
-      gam[0] = 8.0 / 15.0; gam[1] = 5.0 / 12.0; gam[2] = 3.0 / 4.0;
-      rom[0] = 0.0; rom[1] = -17.0 / 60.0; rom[2] = -5.0 / 12.0;
-    } else {
-      gam[0] = 1.5; gam[1] = 0.0; gam[2] = 0.0;
-      rom[0] = -0.5; rom[1] = 0.0; rom[2] = 0.0;
-    }
-    const double dt = S->dt;
-    const double al = gam[ns] + rom[ns];
-    const double beta = dt / B.ren * 0.5;     // TimeMarcher.F90:22
-    S->rk[ns] = BoxScalars::Rk{al, gam[ns], rom[ns], beta};
-    s_bx[SYS_X] = beta * al;
-    s_bx[SYS_YZ] = beta * al;
-    s_bx[SYS_T] = 0.5 * al * dt / B.pec;     // SolveImpEqnUpdate_Temp.F90:25
-  }
-  __syncthreads();
   const int nx = B.nx, nxm = B.nxm;
   // row scale, sub- and super-diagonal (stored temporarily in C_FACT / C_DU)
   for (int t = threadIdx.x; t < 3 * nx; t += blockDim.x) {
@@ -404,7 +407,7 @@ __global__ void __launch_bounds__(K1Shape<TI>::NT, MINB) k_explicit_implicit_fwd
   const long long col = (long long)i * nym + j;
   const int nx = B.nx, nxm = B.nxm;
   const StencilConst c = make_sconst(B);
-  const double al = S->rk[ns].al, ga = S->rk[ns].ga, ro = S->rk[ns].ro, dt = S->dt;
+  const double al = S->rk[1 + ns].al, ga = S->rk[1 + ns].ga, ro = S->rk[1 + ns].ro, dt = S->dt;
   const double alre = al / B.ren;
   const double alpec = al / B.pec;
   const double udy_al = B.dy * al;
@@ -806,10 +809,10 @@ __global__ void __launch_bounds__(256) k_correct(BatchDev bt, int ns, int do_vel
   double *__restrict__ vy = B.vy + col;
   double *__restrict__ vz = B.vz + col;
   double *__restrict__ pr = B.pr + col;
-  const double al = S->rk[ns].al, dt = S->dt;
+  const double al = S->rk[1 + ns].al, dt = S->dt;
   const double udy = al * dt * B.dy;
   const double udz = al * dt * B.dz;
-  const double be = al * S->rk[ns].beta;
+  const double be = al * S->rk[1 + ns].beta;
   const double dzq = B.dzq, dyq = B.dyq;
   const int ke = SEG ? min(ks + kseg, nxm) : nxm;
   double fm = phi[SEG ? (long long)max(ks - 1, 0) * P : 0];   // phi(kmv(k)): phi(0) for k = 0
@@ -896,7 +899,7 @@ __global__ void __launch_bounds__(256, 2) k_divergence(BatchDev bt, int ns, int 
   const double *__restrict__ vy = B.vy + col;
   const double *__restrict__ vz = B.vz + col;
   double *__restrict__ phi = B.phi + col;
-  const double usdtal = 1.0 / (S->dt * S->rk[ns].al);
+  const double usdtal = 1.0 / (S->dt * S->rk[1 + ns].al);
   const double dz = B.dz, dy = B.dy;
   const double *__restrict__ t_udx3m = B.tab + (long long)T_UDX3M * B.nx;   // resolved before the stores
   const int ke = SEG ? min(ks + kseg, nxm) : nxm;

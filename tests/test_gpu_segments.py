@@ -117,6 +117,17 @@ def test_pressure_solve_forms_agree(ctx):
         ctx.remove_box(x)
 
 
+def _check_divergence(box, s, al, dt):
+    """CalcLocalDivergence of s.vy alone uses the coefficient al."""
+    box.upload("vy", s.vy)
+    for f in ("vx", "vz"):
+        box.upload(f, np.zeros_like(s.vy))
+    box.calc_local_divergence()
+    t = O.State(**{**s.__dict__, "vx": np.zeros_like(s.vx), "vz": np.zeros_like(s.vz), "dph": s.dph.copy()})
+    O.calc_local_divergence(t, al, dt)
+    assert np.array_equal(box.download("dph"), t.dph)
+
+
 @pytest.mark.parametrize("nsst,ns", [(3, 0), (3, 2), (1, 0)])
 def test_routines_use_the_substep_prepared_last(ctx, nsst, ns):
     """A step prepares its substeps together; a routine called on its own uses
@@ -128,14 +139,7 @@ def test_routines_use_the_substep_prepared_last(ctx, nsst, ns):
     al = O.init_time_march_scheme(nsst)[2]
     box = _boxes(ctx, [cfg])[0]
 
-    def div(a):
-        box.upload("vy", s.vy)
-        for f in ("vx", "vz"):
-            box.upload(f, np.zeros_like(s.vy))
-        box.calc_local_divergence()
-        t = O.State(**{**s.__dict__, "vx": np.zeros_like(s.vx), "vz": np.zeros_like(s.vz), "dph": s.dph.copy()})
-        O.calc_local_divergence(t, a, cfg.dt)
-        assert np.array_equal(box.download("dph"), t.dph)
+    div = lambda a: _check_divergence(box, s, a, cfg.dt)
 
     ctx.step([box], 1)
     div(al[nsst - 1])
@@ -145,4 +149,33 @@ def test_routines_use_the_substep_prepared_last(ctx, nsst, ns):
     div(al[nsst - 1])
     ctx.step([box], 1, graph=True)
     div(al[nsst - 1])
+    ctx.remove_box(box)
+
+
+def test_a_skipped_preparation_leaves_the_substep(ctx):
+    """Boxes that have failed or are on hold are skipped by steps and by
+    begin_substep alike, so the substep prepared before stays the one that the
+    routines use."""
+    cfg = cfg_of(9, 10, 12, dt=1e-3)
+    s = oracle_state(cfg, seed=2)
+    s.vy[:9] = np.random.default_rng(1).standard_normal((9, 10, 12))
+    al = O.init_time_march_scheme(3)[2]
+    box = _boxes(ctx, [cfg])[0]
+
+    div = lambda a: _check_divergence(box, s, a, cfg.dt)
+
+    box.time_marcher_begin_substep(1)
+    box.upload("vy", 1e6 * s.vy)
+    ctx.step([box], 1)                      # CFL too large: no substep is prepared
+    assert box.scalars()["status"] == 165
+    box.reset()
+    div(al[1])
+    for f in FIELDS:
+        box.upload(f, getattr(oracle_state(cfg, seed=2), f))
+    box.set_stop(1, 0.0, 0.0)
+    ctx.step([box], 1)
+    assert box.scalars()["status"] == 1     # on hold after its step
+    box.time_marcher_begin_substep(0)
+    box.resume()
+    div(al[2])
     ctx.remove_box(box)
