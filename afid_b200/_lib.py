@@ -41,7 +41,7 @@ EXPORTS = [
     "afid_global_quantities", "afid_calc_stats", "afid_calc_dissipation_nu", "afid_box_get_stats",
     "afid_box_reset_stats", "afid_slab_locations", "afid_slab_dump", "afid_box_set_time",
     "afid_box_interp_field", "afid_box_set_stop", "afid_box_resume",
-    "afid_box_test_skip_z_copies", "afid_fft_tile_shape",
+    "afid_box_test_skip_z_copies", "afid_fft_tile_shape", "afid_set_forms",
 ]
 
 STATS = ["vx_me", "vy_me", "vz_me", "temp_me", "vx_rms", "vy_rms", "vz_rms", "temp_rms", "tempvx_me",
@@ -82,6 +82,11 @@ class BoxScalars(C.Structure):
 
 class TileShape(C.Structure):
     _fields_ = [(n, C.c_int) for n in ("y_tile", "z_tile", "y_pairs", "z_lines", "z_rows", "z_slot")]
+
+
+class Forms(C.Structure):
+    _fields_ = [(n, C.c_int) for n in ("y_tile", "z_tile", "k1_variant", "implicit_on_chip", "poisson_on_chip",
+                                       "column_segments", "diag_segments")]
 
 
 class StepRecord(C.Structure):
@@ -136,6 +141,7 @@ def lib(path: str | None = None) -> C.CDLL:
         "afid_step_profiled": ([vp, ip, i, i, dp, ip, i], i),
         "afid_solve_pressure_correction_noalloc": ([vp, i, i, i, dp, d, d, d, vp, ip], i),
         "afid_box_set_tuning": ([vp, i, i, i, i], i),
+        "afid_set_forms": ([vp, ip, i, i, C.POINTER(Forms)], i),
         "afid_fft_tile_shape": ([i, i, i, i, C.POINTER(TileShape)], i),
         "afid_global_quantities": ([vp, i, C.POINTER(GlobalQ)], i),
         "afid_calc_stats": ([vp, i], i),

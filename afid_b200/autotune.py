@@ -4,12 +4,16 @@ For each box size class (nxm, nym, nzm) the tuner times candidate launch
 shapes of the kernels whose shape is free, with device events around every
 kernel (afid_step_profiled), and keeps the fastest:
 
-* row pairs per y-FFT block (forward and inverse y transforms),
-* ky columns per z-FFT block (forward and inverse z transforms),
-* the variant of the explicit/forward kernel: 32x8-column tiles with 2
-  resident blocks (up to 128 registers per thread), with 3 (up to 80), or
-  with two x-planes per barrier; 32x4 tiles with 4, 5 or 6 blocks; 32x2
+* row pairs per tile of the y transforms' tile kernels,
+* ky columns per tile of the z transforms' tile kernels,
+* the variant of the explicit/forward kernel's column form: 32x8-column tiles
+  with 2 resident blocks (up to 128 registers per thread), with 3 (up to 80),
+  or with two x-planes per barrier; 32x4 tiles with 4, 5 or 6 blocks; 32x2
   tiles with 8 blocks.
+
+Only what a launch of the boxes takes is timed (``Context.forms``): lines in
+two register passes have no tiles, and a small set's implicit systems are
+solved on chip without a variant.  The other choices stay 0, the built-in ones.
 
 ``tune`` tunes each size class on a box of its own (for single boxes);
 ``tune_batch`` tunes a set of boxes that are stepped together, on the set.
@@ -119,21 +123,24 @@ def tune_class(ctx, cfg: BouIn, steps: int = 2) -> dict:
         for k, v in initial_fields(cfg, box.xc, seed=0).items():
             box.upload(k, v)
         ctx.step([box], 1)
-        cand = candidates(cfg)
-        best = {}
+        cand, acts = candidates(cfg), ctx.forms([box])
         res = {}
-        for fy in cand["fft_y_lines"]:
-            box.set_tuning(fy, 0, 2)
-            res[("y", fy)] = _time(ctx, box, ("fft_y_fwd", "fft_y_inv"), steps)
-        fy = min(cand["fft_y_lines"], key=lambda v: res[("y", v)])
-        for fz in cand["fft_z_lines"]:
-            box.set_tuning(fy, fz, 2)
-            res[("z", fz)] = _time(ctx, box, ("fft_z_fwd", "fft_z_inv"), steps)
-        fz = min(cand["fft_z_lines"], key=lambda v: res[("z", v)])
-        for mb in cand["k1_minb"]:
-            box.set_tuning(fy, fz, mb)
-            res[("k1", mb)] = _time(ctx, box, ("explicit_fwd",), steps)
-        mb = min(cand["k1_minb"], key=lambda v: res[("k1", v)])
+        fy = fz = mb = 0
+        if acts["y_tile"]:
+            for v in cand["fft_y_lines"]:
+                box.set_tuning(v, 0, 2)
+                res[("y", v)] = _time(ctx, box, ("fft_y_fwd", "fft_y_inv"), steps)
+            fy = min(cand["fft_y_lines"], key=lambda v: res[("y", v)])
+        if acts["z_tile"]:
+            for v in cand["fft_z_lines"]:
+                box.set_tuning(fy, v, 2)
+                res[("z", v)] = _time(ctx, box, ("fft_z_fwd", "fft_z_inv"), steps)
+            fz = min(cand["fft_z_lines"], key=lambda v: res[("z", v)])
+        if acts["k1_variant"]:
+            for v in cand["k1_minb"]:
+                box.set_tuning(fy, fz, v)
+                res[("k1", v)] = _time(ctx, box, ("explicit_fwd",), steps)
+            mb = min(cand["k1_minb"], key=lambda v: res[("k1", v)])
         best = {"fft_y_lines": fy, "fft_z_lines": fz, "k1_minb": mb,
                 "ms_per_step": {f"{a}{b}": round(t / steps, 4) for (a, b), t in res.items()}}
         return best
@@ -184,21 +191,24 @@ def tune_batch(ctx, boxes, steps: int = 2) -> dict:
 
     res = {}
     set_all(0, 0, 0)
-    res[("y", 0)] = t(("fft_y_fwd", "fft_y_inv"))
-    for fy in y_all:
-        set_all(fy, 0, 0)
-        res[("y", fy)] = t(("fft_y_fwd", "fft_y_inv"))
-    fy = min([0] + y_all, key=lambda v: res[("y", v)])
-    set_all(fy, 0, 0)
-    res[("z", 0)] = t(("fft_z_fwd", "fft_z_inv"))
-    for fz in z_all:
-        set_all(fy, fz, 0)
-        res[("z", fz)] = t(("fft_z_fwd", "fft_z_inv"))
-    fz = min([0] + z_all, key=lambda v: res[("z", v)])
-    for mb in candidates(boxes[0].cfg)["k1_minb"]:
-        set_all(fy, fz, mb)
-        res[("k1", mb)] = t(("explicit_fwd",))
-    mb = min(candidates(boxes[0].cfg)["k1_minb"], key=lambda v: res[("k1", v)])
+    acts = ctx.forms(boxes)
+    fy = fz = mb = 0
+    if acts["y_tile"]:
+        for v in [0] + y_all:
+            set_all(v, 0, 0)
+            res[("y", v)] = t(("fft_y_fwd", "fft_y_inv"))
+        fy = min([0] + y_all, key=lambda v: res[("y", v)])
+    if acts["z_tile"]:
+        for v in [0] + z_all:
+            set_all(fy, v, 0)
+            res[("z", v)] = t(("fft_z_fwd", "fft_z_inv"))
+        fz = min([0] + z_all, key=lambda v: res[("z", v)])
+    if acts["k1_variant"]:
+        variants = candidates(boxes[0].cfg)["k1_minb"]
+        for v in variants:
+            set_all(fy, fz, v)
+            res[("k1", v)] = t(("explicit_fwd",))
+        mb = min(variants, key=lambda v: res[("k1", v)])
     set_all(fy, fz, mb)
     return {"fft_y_lines": fy, "fft_z_lines": fz, "k1_minb": mb,
             "ms_per_step": {f"{a}{b}": round(v, 4) for (a, b), v in res.items()}}

@@ -1930,6 +1930,29 @@ int split_halves(afid_ctx *c, const Batch *bt, Batch **hb) {
 
 extern "C" {
 
+int afid_set_forms(afid_ctx *c, const int *ids, int n, int part, afid_forms *out) {
+  if (!c || !out) return fail(AFID_EINVAL, "null argument");
+  int rc = set_device(c);
+  if (rc) return rc;
+  Batch *bt;
+  rc = get_batch(c, ids, n, &bt);
+  if (rc) return rc;
+  if (part) {
+    if (part < 0 || part > 2 || !bt->split) return fail(AFID_EINVAL, "set_forms: part %d of a set that is not split", part);
+    const std::vector<int> &h = bt->half_ids[part - 1];
+    rc = get_batch(c, h.data(), (int)h.size(), &bt, false);
+    if (rc) return rc;
+  }
+  out->y_tile = bt->total[FAM_FY] > 0;
+  out->z_tile = bt->total[FAM_FZ] > 0;
+  out->k1_variant = bt->total[FAM_K1] > 0 ? bt->k1_minb : 0;
+  out->implicit_on_chip = bt->total[FAM_KS] > 0;
+  out->poisson_on_chip = bt->smem_px > 0;
+  out->column_segments = bt->nseg;
+  out->diag_segments = bt->nseg;
+  return 0;
+}
+
 int afid_step_graph(afid_ctx *c, const int *ids, int n, int nsteps) {
   if (!c) return fail(AFID_EINVAL, "null ctx");
   if (nsteps < 0) return fail(AFID_EINVAL, "nsteps < 0");

@@ -138,6 +138,14 @@ class Context:
         _lib.check(self._L.afid_step_graph_kernels(self.h, ids, n, C.byref(k)))
         return k.value
 
+    def forms(self, boxes, part: int = 0) -> dict:
+        """Forms that the kernels of a step of ``boxes`` take: whole (part 0)
+        or as one of the halves (1, 2) of a split graph step."""
+        ids, n = self._ids(boxes)
+        f = _lib.Forms()
+        _lib.check(self._L.afid_set_forms(self.h, ids, n, part, C.byref(f)))
+        return {k: getattr(f, k) for k, _ in f._fields_}
+
     def scalars(self, boxes) -> list[dict]:
         """Box.scalars() of every box of ``boxes``, read with one copy."""
         ids, n = self._ids(boxes)

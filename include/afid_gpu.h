@@ -209,7 +209,10 @@ int afid_box_test_skip_z_copies(afid_ctx *ctx, int box_id, int skip, unsigned ma
  * 2 = 32x8-column tiles, two resident blocks per SM; 3 = 32x8, three
  * resident blocks; 4 = 32x8, two planes per barrier; 5, 7, 8 = 32x4 tiles,
  * four, five or six blocks; 6 = 32x2 tiles, eight blocks (0 = 4).  Results
- * do not depend on these values. */
+ * do not depend on these values.  They are kept for every box, and act where
+ * its launches take them (afid_set_forms): the lines on transforms in the tile
+ * kernels, the variant in sets large enough for the explicit kernel's column
+ * form. */
 int afid_box_set_tuning(afid_ctx *ctx, int box_id, int fft_y_lines, int fft_z_lines, int k1_minb);
 /* Transform tiles of nym x nzm lines with the given lines per tile (as
  * afid_box_set_tuning takes them; host only, no counterpart in the reference). */
@@ -220,6 +223,18 @@ typedef struct afid_tile_shape {
   int z_slot;           /* complex values from one z slot in shared memory to the next */
 } afid_tile_shape;
 int afid_fft_tile_shape(int nym, int nzm, int fft_y_lines, int fft_z_lines, afid_tile_shape *out);
+/* Forms that the kernels of a step of this box set take (no counterpart in the
+ * reference; the results do not depend on them): of the whole set (part 0), or of one
+ * of the halves (1, 2) that afid_step_graph runs a large set as. */
+typedef struct afid_forms {
+  int y_tile, z_tile;     /* 1: some boxes' lines run in the tile kernels */
+  int k1_variant;         /* of the explicit/forward kernel's column form, 0: no box runs it */
+  int implicit_on_chip;   /* 1: some boxes' implicit systems are solved with the columns on chip */
+  int poisson_on_chip;    /* 1: the pressure's x-solve runs with the modes' columns on chip */
+  int column_segments;    /* segments of planes of the divergence and the correction */
+  int diag_segments;      /* and of the diagnostics */
+} afid_forms;
+int afid_set_forms(afid_ctx *ctx, const int *box_ids, int nbox, int part, afid_forms *out);
 /* Copies up to max_records of the most recent per-step records, oldest
  * first; returns the number copied (>= 0) or an error code. */
 int afid_box_history(afid_ctx *ctx, int box_id, afid_step_record *out, int max_records);
@@ -266,7 +281,7 @@ int afid_substep(afid_ctx *ctx, const int *box_ids, int nbox, int ns);
 /* Kernel slots of afid_step_profiled. */
 enum afid_kernel {
   AFID_K_DIAG = 0,          /* CalcMaxCFL + CheckDivergence + vmax reduction */
-  AFID_K_FINALIZE = 1,      /* dt rule / step bookkeeping */
+  AFID_K_FINALIZE = 1,      /* 0: the dt rule and the step's bookkeeping run in AFID_K_DIAG and AFID_K_PLATE_NU */
   AFID_K_PREP = 2,          /* substep coefficients and x-tridiagonal LU */
   AFID_K_EXPLICIT_FWD = 3,  /* ExplicitTerms* + ImplicitAndUpdate* rhs + forward sweeps */
   AFID_K_IMPLICIT_BWD = 4,  /* back substitution + update of vx, vy, vz, temp */

@@ -18,9 +18,15 @@ MIX = [
 ]
 
 
+# lines in the tile kernels of the transforms, and a box whose column tiles
+# (157) put a set that holds it on the explicit kernel's column form
+TILES = dict(nxm=12, nym=56, nzm=42, ray=1e5, pra=0.7, ylen=1.0, zlen=0.9, dt=2e-4)
+FILLER = dict(nxm=6, nym=200, nzm=200, dt=1e-4)
+
+
 def _add(ctx, kw, seed):
     cfg = cfg_of(**kw)
-    b = ctx.add_box(cfg)
+    b = ctx.add_box(cfg, validate=False)
     for k, v in initial_fields(cfg, b.xc, seed).items():
         b.upload(k, v)
     return b
@@ -41,6 +47,19 @@ def test_batch_equals_alone_and_graph_equals_direct(ctx):
             assert np.array_equal(fa, fg), f
         assert a.scalars() == b.scalars()
     for b in batch + alone + graphed:
+        ctx.remove_box(b)
+
+
+def test_only_shapes_that_act_are_tuned(ctx):
+    """A small set with two-pass lines takes no launch shape: the tuner times
+    none and leaves the built-in choices."""
+    from afid_b200 import autotune
+    boxes = [_add(ctx, kw, q) for q, kw in enumerate(MIX)]
+    f = ctx.forms(boxes)
+    assert (f["y_tile"], f["z_tile"], f["k1_variant"], f["implicit_on_chip"]) == (0, 0, 0, 1)
+    assert autotune.tune_batch(ctx, boxes, steps=1) == {"fft_y_lines": 0, "fft_z_lines": 0, "k1_minb": 0,
+                                                        "ms_per_step": {}}
+    for b in boxes:
         ctx.remove_box(b)
 
 
@@ -99,18 +118,21 @@ def test_launch_shapes_do_not_change_results(ctx, fy, fz, k1):
     """Tuned launch shapes (FFT lines per block, tile shape and occupancy of
     the explicit kernel) give bit-identical fields to the defaults (explicit
     kernel variant 4)."""
-    a = _add(ctx, MIX[2], 21)
-    b = _add(ctx, MIX[2], 21)
-    b.set_tuning(fft_y_lines=fy, fft_z_lines=fz, k1_minb=k1)
-    ctx.step([a], 3)
-    ctx.step([b], 3)
-    for f in FIELDS:
-        assert np.array_equal(a.download(f), b.download(f)), f
+    sets = [[_add(ctx, kw, 21) for kw in (TILES, MIX[2], FILLER)] for _ in range(2)]
+    for x in sets[1]:
+        x.set_tuning(fft_y_lines=fy, fft_z_lines=fz, k1_minb=k1)
+    acts = [ctx.forms(s) for s in sets]
+    assert [(f["y_tile"], f["z_tile"], f["k1_variant"]) for f in acts] == [(1, 1, 4), (1, 1, k1)]
+    for s in sets:
+        ctx.step(s, 3)
+    for a, b in zip(*sets):
+        for f in FIELDS:
+            assert np.array_equal(a.download(f), b.download(f)), f
     from afid_b200._lib import AfidError
     for bad in (dict(fft_y_lines=10 ** 6), dict(fft_y_lines=3), dict(fft_z_lines=6), dict(k1_minb=9)):
         with pytest.raises(AfidError):
-            b.set_tuning(**bad)
-    for x in (a, b):
+            sets[1][1].set_tuning(**bad)
+    for x in sets[0] + sets[1]:
         ctx.remove_box(x)
 
 
@@ -118,11 +140,13 @@ def test_batch_tuning_keeps_results(ctx):
     """autotune.tune_batch chooses the launch shapes on the set itself; the
     chosen shapes change no result bit."""
     from afid_b200 import autotune
-    tuned = [_add(ctx, kw, 20 + q) for q, kw in enumerate(MIX)]
-    plain = [_add(ctx, kw, 20 + q) for q, kw in enumerate(MIX)]
+    kws = MIX + [TILES, FILLER]
+    tuned = [_add(ctx, kw, 20 + q) for q, kw in enumerate(kws)]
+    plain = [_add(ctx, kw, 20 + q) for q, kw in enumerate(kws)]
     choice = autotune.tune_batch(ctx, tuned, steps=1)
     assert choice["k1_minb"] in autotune.candidates(tuned[0].cfg)["k1_minb"]
-    for b, kw, q in zip(tuned, MIX, range(len(MIX))):        # restart from the seeded state
+    assert {k[0] for k in choice["ms_per_step"]} == {"y", "z", "k"}
+    for b, kw, q in zip(tuned, kws, range(len(kws))):        # restart from the seeded state
         for k, v in initial_fields(b.cfg, b.xc, 20 + q).items():
             b.upload(k, v)
         b.reset(b.cfg.dt)

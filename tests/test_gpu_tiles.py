@@ -5,7 +5,7 @@ use both shared-memory slots."""
 import numpy as np
 import pytest
 
-from helpers import cfg_of, oracle_state, rel_l2
+from helpers import cfg_of, oracle_state, rel_l2, FIELDS
 from oracle import afid_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -46,3 +46,33 @@ def test_z_tiles_in_both_slots(ctx, nxm, nym, nzm, fz):
     got, s = _solve(ctx, cfg_of(nxm, nym, nzm, ylen=1.3, zlen=0.9, istr3=0), 0, fz)
     O.solve_pressure_correction(s)
     assert rel_l2(got, s.dph, remove_mean=True) <= 1e-11
+
+
+@pytest.mark.parametrize("fy,fz", [(0, 0), (1, 1), (4, 2)])
+def test_tile_boxes_in_a_set(ctx, fy, fz):
+    """Boxes of different tile lines in one launch of each transform come out
+    as each does alone with the built-in lines per tile."""
+    cfgs = [cfg_of(12, 56, 42, dt=2e-4, ylen=1.2), cfg_of(5, 14, 441, dt=1e-4), cfg_of(9, 98, 21, dt=2e-4),
+            cfg_of(4, 1152, 28, dt=1e-5), cfg_of(7, 10, 972, dt=1e-5)]
+
+    def boxes():
+        out = []
+        for q, cfg in enumerate(cfgs):
+            s = oracle_state(cfg, seed=q)
+            out.append(ctx.add_box(cfg, s.g.xc, validate=False))
+            for f in FIELDS:
+                out[-1].upload(f, getattr(s, f))
+        return out
+
+    alone, batch = boxes(), boxes()
+    for b in alone:
+        ctx.step([b], 2)
+    for b in batch:
+        b.set_tuning(fy if b.cfg.nym * fy <= 3584 else 0, fz, 0)
+    ctx.step(batch, 2)
+    for a, b in zip(alone, batch):
+        assert b.scalars()["status"] == 0
+        for f in FIELDS:
+            assert np.array_equal(a.download(f), b.download(f)), f
+    for b in alone + batch:
+        ctx.remove_box(b)
