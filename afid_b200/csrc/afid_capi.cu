@@ -150,6 +150,7 @@ int two_pass_class(const int *r) { return !r[0] ? -1 : r[1] > 16 ? 1 : 0; }
 //   5: 32x4 tiles, 4 blocks/SM        6: 32x2 tiles, 8 blocks/SM
 //   7: 32x4 tiles, 5 blocks/SM        8: 32x4 tiles, 6 blocks/SM
 constexpr int ON_CHIP_SMEM = 226 * 1024;   // most shared memory of k_implicit_cols and k_poisson_cols
+constexpr int SM_SMEM = 228 * 1024;        // of an SM, 1 KB of it reserved for each block
 constexpr int K1_VMIN = 2, K1_VMAX = 8;
 constexpr int K1_DEFAULT = 4;   // the variant the tuner picks for the large boxes (768^2, 1280^2)
 int k1_tile_height(int variant) { return (variant == 5 || variant >= 7) ? 4 : variant == 6 ? 2 : 8; }
@@ -492,18 +493,29 @@ void plane_segments(int nsm, int tiles, int nxm, int *kseg, int *nseg) {
 // systems on chip: K1 writes right-hand sides, k_implicit_cols does both
 // sweeps.  K1 + K2 per step: 75x150x135 (80 tiles) 0.48 -> 0.33 ms; twelve
 // ensemble boxes (about 330 tiles) 1.02 -> 1.12 ms, so the line lies between.
+// Tall boxes meet it earlier: the column kernels take one wave whatever the
+// tiles, k_implicit_cols as many as its blocks need at the ``fit`` blocks that
+// an SM's shared memory holds, each wave of them longer the more it holds.  Column
+// over on-chip time of K1 + K2 against the rounds x (fit + 2) that the rule bounds by
+// 22: 1.19 at 21 (200 to 400 x 128^2), 1.09 at 22 (160^3), 0.97 at 22
+// (152x162^2), 0.96 at 23 (123x180^2), 0.87 at 31 (160x192^2), 0.80 at 32 (256x160^2)
+// and 0.59 at 47 (256 to 400 x 192^2).
 // Boxes too tall for a block's shared memory (nxm > 401) keep the column
 // kernels.  Results do not depend on the choice.  Returns the shared memory of
 // the k_implicit_cols launch.
 size_t choose_on_chip(int nsm, std::vector<BoxDev> &devs) {
-  long long tiles = 0;
-  for (const BoxDev &d : devs) tiles += cdiv(d.plane, 256);
+  long long tiles = 0, blocks = 0;
   size_t smem = 0;
-  for (BoxDev &d : devs) {
-    d.on_chip = tiles < nsm && ks_bytes(d.nxm) <= ON_CHIP_SMEM;
-    if (d.on_chip) smem = std::max(smem, (size_t)ks_bytes(d.nxm));
+  for (const BoxDev &d : devs) {
+    tiles += cdiv(d.plane, 256);
+    if (ks_bytes(d.nxm) > ON_CHIP_SMEM) continue;
+    blocks += 2 * cdiv(d.plane, KS_COLS);
+    smem = std::max(smem, (size_t)ks_bytes(d.nxm));
   }
-  return smem;
+  const long long fit = SM_SMEM / (long long)(smem + 1024);
+  const bool on = tiles < nsm && blocks * (fit + 2) < 22LL * nsm * fit;
+  for (BoxDev &d : devs) d.on_chip = on && ks_bytes(d.nxm) <= ON_CHIP_SMEM;
+  return on ? smem : 0;
 }
 
 // Shared memory of the on-chip x-solve (k_poisson_cols) for a set of ``warps``

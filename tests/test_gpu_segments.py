@@ -73,6 +73,17 @@ def test_on_chip_and_column_solves_agree(ctx, k1):
         ctx.remove_box(b)
 
 
+@pytest.mark.parametrize("nxm,n,on_chip", [(24, 16, 1), (64, 192, 1), (400, 96, 1), (400, 128, 1), (150, 160, 1),
+                                           (256, 160, 0), (160, 192, 0), (256, 192, 0), (404, 16, 0), (16, 196, 0)])
+def test_on_chip_solves_where_their_waves_are_few(ctx, nxm, n, on_chip):
+    """256x192^2 needs 16 waves of on-chip blocks (1 per SM) and took 5% longer
+    per step than with the column kernels."""
+    box = ctx.add_box(cfg_of(nxm, n, n, dt=1e-5), validate=False)
+    f = ctx.forms([box])
+    assert f["implicit_on_chip"] == on_chip and (f["k1_variant"] == 0) == bool(on_chip)
+    ctx.remove_box(box)
+
+
 @pytest.mark.parametrize("nxm", [4, 9, 33, 400, 404])
 def test_on_chip_solves_match_oracle(ctx, nxm):
     """nxm = 400 is near the tallest on-chip column, 404 is beyond it."""
