@@ -494,16 +494,18 @@ void plane_segments(int nsm, int tiles, int nxm, int *kseg, int *nseg) {
 // sweeps.  K1 + K2 per step: 75x150x135 (80 tiles) 0.48 -> 0.33 ms; twelve
 // ensemble boxes (about 330 tiles) 1.02 -> 1.12 ms, so the line lies between.
 // Tall boxes meet it earlier: the column kernels take one wave whatever the
-// tiles, k_implicit_cols as many as its blocks need at the ``fit`` blocks that
-// an SM's shared memory holds, each wave of them longer the more it holds.  Column
-// over on-chip time of K1 + K2 against the rounds x (fit + 2) that the rule bounds by
-// 22: 1.19 at 21 (200 to 400 x 128^2), 1.09 at 22 (160^3), 0.97 at 22
-// (152x162^2), 0.96 at 23 (123x180^2), 0.87 at 31 (160x192^2), 0.80 at 32 (256x160^2)
-// and 0.59 at 47 (256 to 400 x 192^2).
+// tiles, k_implicit_cols as many as its blocks need at the ``fit`` blocks that an
+// SM's shared memory holds, each wave of them longer the more it holds.  The rule
+// bounds blocks per SM x (fit + 2) / fit by 22.  K1 + K2 per step, column kernels
+// against on chip: 100x180^2 (23) 0.63 and 0.67 ms, 160x192^2 (31) 0.98 and 1.22,
+// 256x160^2 (32) 1.49 and 2.05, 400x192^2 (47) 2.36 and 4.31; below it, the column
+// kernels timed before their divisions went, 160^3 (22) 1.04 and 0.95, 256x128^2
+// (21) 1.60 and 1.35.
 // Boxes too tall for a block's shared memory (nxm > 401) keep the column
 // kernels.  Results do not depend on the choice.  Returns the shared memory of
 // the k_implicit_cols launch.
-size_t choose_on_chip(int nsm, std::vector<BoxDev> &devs) {
+// A half of a split set does as the set would whole.
+size_t choose_on_chip(int nsm, std::vector<BoxDev> &devs, const Batch *whole) {
   long long tiles = 0, blocks = 0;
   size_t smem = 0;
   for (const BoxDev &d : devs) {
@@ -513,23 +515,23 @@ size_t choose_on_chip(int nsm, std::vector<BoxDev> &devs) {
     smem = std::max(smem, (size_t)ks_bytes(d.nxm));
   }
   const long long fit = SM_SMEM / (long long)(smem + 1024);
-  const bool on = tiles < nsm && blocks * (fit + 2) < 22LL * nsm * fit;
+  const bool on = whole ? whole->smem_ks > 0 : tiles < nsm && blocks * (fit + 2) < 22LL * nsm * fit;
   for (BoxDev &d : devs) d.on_chip = on && ks_bytes(d.nxm) <= ON_CHIP_SMEM;
   return on ? smem : 0;
 }
 
 // Shared memory of the on-chip x-solve (k_poisson_cols) for a set of ``warps``
 // groups of 32 modes and at most nxm planes, or 0 for k_poisson_x: on chip up
-// to four rounds of the warps the SMs hold, in a half of a split set (whose
-// other half runs beside it) up to two.  Per step, on chip against k_poisson_x:
+// to four rounds of the warps the SMs hold.  Per step, on chip against k_poisson_x:
 // 65x64x64 (0.1 rounds) 0.042 and 0.129 ms, 48x384x243 (1.1) 0.081 and 0.123,
 // twelve ensemble boxes (2.4) 0.123 and 0.223, 24 (4.1) 0.227 and 0.279, 64
-// (11) 0.497 and 0.492, 192x384x384 (7.8) 0.80 and 0.61; whole steps of split
-// sets, 20 boxes (halves of 1.8 rounds) 3.24 and 3.32, 24 (2.0) 3.75 and 3.64.
+// (11) 0.497 and 0.492, 192x384x384 (7.8) 0.80 and 0.61.  Not in a half of a
+// split set, whose other half runs beside it: there its shared memory keeps the
+// other half's blocks off the SMs.
 size_t px_cols_smem(int nsm, int warps, int nxm, bool half) {
   const int bytes = px_cols_bytes(nxm);
-  if (bytes > ON_CHIP_SMEM) return 0;
-  return warps <= (half ? 2LL : 4LL) * nsm * (ON_CHIP_SMEM / bytes) ? (size_t)bytes : 0;
+  if (half || bytes > ON_CHIP_SMEM) return 0;
+  return warps <= 4LL * nsm * (ON_CHIP_SMEM / bytes) ? (size_t)bytes : 0;
 }
 
 // Planes per block of the K1 launch of such a set (one block per SM): the
@@ -546,16 +548,23 @@ void k1s_segments(int nsm, int tiles, int nxm, int *kseg, int *nseg) {
   }
 }
 
-int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split = true) {
+// The batch of a box set or, with ``whole``, of the half of a split one.  Halves run
+// side by side, so the forms of their launches follow from the whole set's size; they
+// are kept apart from a set that a caller steps by itself.
+int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, const Batch *whole = nullptr) {
   if (n <= 0 || !ids) return fail(AFID_EINVAL, "empty box set");
   std::vector<int> key(ids, ids + n);
+  if (whole) {
+    key.push_back(-1);
+    key.insert(key.end(), whole->ids.begin(), whole->ids.end());
+  }
   auto it = c->batches.find(key);
   if (it != c->batches.end()) { *out = it->second; return 0; }
   std::vector<BoxDev> devs;
   std::vector<int> off((size_t)NFAM * (n + 1), 0);
   Batch *bt = new Batch();
   int twy_max = 0, twz_max = 0;
-  bt->ids = key;
+  bt->ids.assign(ids, ids + n);
   for (int b = 0; b < n; ++b) {
     HostBox *hb;
     int rc = get_box(c, ids[b], &hb);
@@ -591,7 +600,7 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
     if (e && atoi(e) >= K1_VMIN && atoi(e) <= K1_VMAX) bt->k1_minb = atoi(e);
   }
   const int nsm = nsm_of_device();
-  bt->smem_ks = choose_on_chip(nsm, devs);
+  bt->smem_ks = choose_on_chip(nsm, devs, whole);
   {
     int rc = k2_block_size(devs, &bt->k2_block);
     if (rc) { delete bt; return rc; }
@@ -607,9 +616,10 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
     bt->total[f] = (int)acc;
   }
   for (const BoxDev &d : devs) bt->nsst = std::max(bt->nsst, d.nsst);
-  bt->smem_px = px_cols_smem(nsm, bt->total[FAM_PXS], devs[0].nxm, !allow_split);
-  plane_segments(nsm, bt->total[FAM_COL], devs[0].nxm, &bt->kseg, &bt->nseg);
-  k1s_segments(nsm, bt->total[FAM_K1S], devs[0].nxm, &bt->k1s_seg, &bt->k1s_nseg);
+  const int *total = whole ? whole->total : bt->total;   // of the launches that share the device
+  bt->smem_px = px_cols_smem(nsm, bt->total[FAM_PXS], devs[0].nxm, whole != nullptr);
+  plane_segments(nsm, total[FAM_COL], devs[0].nxm, &bt->kseg, &bt->nseg);
+  k1s_segments(nsm, total[FAM_K1S], devs[0].nxm, &bt->k1s_seg, &bt->k1s_nseg);
   off.insert(off.end(), pos.begin(), pos.end());   // the positions follow the tile tables
   if (cudaMalloc(&bt->d_boxes, sizeof(BoxDev) * n) != cudaSuccess ||
       cudaMalloc(&bt->d_off, sizeof(int) * off.size()) != cudaSuccess) {
@@ -625,7 +635,7 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, bool allow_split 
     if (!rc) rc = f2_shapes(devs, bt->total, bt->f2);
     if (rc) { free_batch(bt); return rc; }
   }
-  if (allow_split && n >= SPLIT_MIN_BOXES) {
+  if (!whole && n >= SPLIT_MIN_BOXES) {
     long long cells = 0;
     for (const BoxDev &d : devs) cells += (long long)d.nxm * d.plane;
     if (cells >= SPLIT_MIN_CELLS) {
@@ -1932,7 +1942,7 @@ int ensure_side(afid_ctx *c) {
 int split_halves(afid_ctx *c, const Batch *bt, Batch **hb) {
   int rc = ensure_side(c);
   for (int h = 0; !rc && h < 2; ++h) {
-    rc = get_batch(c, bt->half_ids[h].data(), (int)bt->half_ids[h].size(), &hb[h], false);
+    rc = get_batch(c, bt->half_ids[h].data(), (int)bt->half_ids[h].size(), &hb[h], bt);
     if (!rc) rc = ensure_graph(hb[h], c->side[h]);
   }
   return rc;
@@ -1952,7 +1962,7 @@ int afid_set_forms(afid_ctx *c, const int *ids, int n, int part, afid_forms *out
   if (part) {
     if (part < 0 || part > 2 || !bt->split) return fail(AFID_EINVAL, "set_forms: part %d of a set that is not split", part);
     const std::vector<int> &h = bt->half_ids[part - 1];
-    rc = get_batch(c, h.data(), (int)h.size(), &bt, false);
+    rc = get_batch(c, h.data(), (int)h.size(), &bt, bt);
     if (rc) return rc;
   }
   out->y_tile = bt->total[FAM_FY] > 0;

@@ -190,3 +190,21 @@ def test_a_skipped_preparation_leaves_the_substep(ctx):
     box.resume()
     div(al[2])
     ctx.remove_box(box)
+
+
+@pytest.mark.parametrize("n,shape", [(8, (64, 96, 96)), (12, (32, 128, 128)), (24, (64, 64, 64))])
+def test_halves_take_the_whole_sets_forms(ctx, n, shape):
+    """The halves of a split set run side by side: each takes the forms that the
+    whole set would, and the x-solve that leaves shared memory to the other
+    half.  A half's boxes stepped by themselves choose for themselves."""
+    boxes = [ctx.add_box(cfg_of(*shape, dt=1e-5)) for _ in range(n)]
+    whole = ctx.forms(boxes)
+    for part in (1, 2):
+        f = ctx.forms(boxes, part)
+        assert f == {**whole, "poisson_on_chip": 0}
+    own = ctx.forms(boxes[::2])
+    assert own["poisson_on_chip"] == 1
+    if n // 2 * shape[1] * shape[2] < 296 * 256:       # fewer column tiles than resident blocks
+        assert own["column_segments"] > whole["column_segments"]
+    for b in boxes:
+        ctx.remove_box(b)
