@@ -89,7 +89,8 @@ struct Batch {
   size_t smem_ks = 0;               // shared memory of k_implicit_cols
   size_t smem_px = 0;               // shared memory of k_poisson_cols (0: the set runs k_poisson_x)
   int nsst = 1;                     // most substeps of its boxes
-  int kseg = 0, nseg = 1;           // planes per block and blocks per column tile of the planewise marches
+  int kseg = 0, nseg = 1;           // planes per block and blocks per column tile of divergence and correction
+  int diag_kseg = 0, diag_nseg = 1; // and of the diagnostics
   F2Shape f2[4];                    // two-pass transforms: y and z of classes 0 and 1
   cudaGraphExec_t gexec = nullptr;
   cudaStream_t gstream = nullptr;
@@ -479,15 +480,25 @@ int nsm_of_device() {
 
 // Planes per block of the marches whose planes are independent (divergence,
 // correction, diagnostics), for a set of ``tiles`` column tiles and at most
-// nxm planes: whole columns once the tiles fill the resident blocks (two per
-// SM), else segments that give each SM two rounds of blocks.
-void plane_segments(int nsm, int tiles, int nxm, int *kseg, int *nseg) {
-  const long long resident = 2LL * nsm;
-  long long n = tiles >= resident ? 1 : cdiv(2 * resident, std::max(tiles, 1));
-  n = std::min(n, cdiv(nxm, KC_U));
+// nxm planes: whole columns from ``limit`` tiles on, else segments that give
+// each SM two rounds of its resident blocks.
+void plane_segments(int nsm, int tiles, int nxm, int limit, int *kseg, int *nseg) {
+  const long long n = tiles >= limit ? 1 : std::min(cdiv(4LL * nsm, std::max(tiles, 1)), cdiv(nxm, KC_U));
   *kseg = (int)(cdiv(cdiv(nxm, n), KC_U) * KC_U);
   *nseg = (int)cdiv(nxm, *kseg);
 }
+
+// Where the segments stop.  Two blocks of 256 columns fit an SM; whole columns run
+// faster per plane (registers, k_stencil.cuh), so segments gain only while the tiles
+// leave a good part of the SMs idle: divergence and correction up to two thirds
+// of the resident blocks, the diagnostics, whose segments lose most, up to one
+// third.  Segments against whole columns, ms per step: correction 0.42 and 0.53
+// on 256x192^2 (144 tiles), 0.28 and 0.31 on 128x216^2 (183), 0.36 and 0.33 on
+// 128x240^2 (225); diagnostics with the dt rule 0.052 and 0.074 on 128x150^2 (88),
+// 0.109 and 0.101 on 256x160^2 (100), 0.134 and 0.103 on 256x192^2, 0.21 and 0.12
+// on 256^3 (256).
+int column_limit(int nsm) { return 4 * nsm / 3; }
+int diag_limit(int nsm) { return 2 * nsm / 3; }
 
 // Small sets (fewer than one block of 256 columns per SM) solve their implicit
 // systems on chip: K1 writes right-hand sides, k_implicit_cols does both
@@ -618,7 +629,8 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, const Batch *whol
   for (const BoxDev &d : devs) bt->nsst = std::max(bt->nsst, d.nsst);
   const int *total = whole ? whole->total : bt->total;   // of the launches that share the device
   bt->smem_px = px_cols_smem(nsm, bt->total[FAM_PXS], devs[0].nxm, whole != nullptr);
-  plane_segments(nsm, total[FAM_COL], devs[0].nxm, &bt->kseg, &bt->nseg);
+  plane_segments(nsm, total[FAM_COL], devs[0].nxm, column_limit(nsm), &bt->kseg, &bt->nseg);
+  plane_segments(nsm, total[FAM_DIAG], devs[0].nxm, diag_limit(nsm), &bt->diag_kseg, &bt->diag_nseg);
   k1s_segments(nsm, total[FAM_K1S], devs[0].nxm, &bt->k1s_seg, &bt->k1s_nseg);
   off.insert(off.end(), pos.begin(), pos.end());   // the positions follow the tile tables
   if (cudaMalloc(&bt->d_boxes, sizeof(BoxDev) * n) != cudaSuccess ||
@@ -820,8 +832,8 @@ void launch_correct(const Batch *bt, cudaStream_t s, int ns, int vel, int pr) {
 }
 
 void launch_diag(const Batch *bt, cudaStream_t s, int every_box) {
-  const dim3 g(bt->total[FAM_DIAG], bt->nseg);
-  if (bt->nseg > 1) k_diag<true><<<g, 256, 0, s>>>(bdev(bt, FAM_DIAG), every_box, bt->kseg);
+  const dim3 g(bt->total[FAM_DIAG], bt->diag_nseg);
+  if (bt->diag_nseg > 1) k_diag<true><<<g, 256, 0, s>>>(bdev(bt, FAM_DIAG), every_box, bt->diag_kseg);
   else k_diag<false><<<g, 256, 0, s>>>(bdev(bt, FAM_DIAG), every_box, 0);
 }
 
@@ -1971,7 +1983,7 @@ int afid_set_forms(afid_ctx *c, const int *ids, int n, int part, afid_forms *out
   out->implicit_on_chip = bt->total[FAM_KS] > 0;
   out->poisson_on_chip = bt->smem_px > 0;
   out->column_segments = bt->nseg;
-  out->diag_segments = bt->nseg;
+  out->diag_segments = bt->diag_nseg;
   return 0;
 }
 
