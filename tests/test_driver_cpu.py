@@ -33,7 +33,7 @@ def test_output_rule_and_wnus_means():
 
 class FakeBox:
     """Applies the device's per-step bookkeeping and hold rules
-    (k_finalize): time += dt, ntime += 1, hold at stop_ntime / output
+    (finalize_box): time += dt, ntime += 1, hold at stop_ntime / output
     times / time > tmax; a planted failure code at a given step."""
 
     def __init__(self, dt, fail_at=None, fail_code=266):

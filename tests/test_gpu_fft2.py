@@ -1,20 +1,42 @@
 """The two-pass transforms (lines of N = r1 r2 points, both radices at most 32)
-through the pressure solve, against the oracle: every radix in either pass, tiles
-with lines beyond the box (odd row counts, ky counts that do not fill a tile),
-and the sizes next to them that the tile kernels keep (a factor of 7, more
-than 1024 points)."""
+through the pressure solve, against the oracle: in y and in z every radix in
+either pass, tiles with lines beyond the box (odd row counts, ky counts that do not
+fill a tile), and lengths that the tile kernels keep (a factor of 7, more than
+1024 points)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
+from afid_b200 import _lib
 from helpers import cfg_of, oracle_state, rel_l2
 from oracle import afid_oracle as O
 
-pytestmark = pytest.mark.gpu
+RADICES = [2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16, 18, 20, 24, 25, 27, 30, 32]
+Y = [4, 6, 10, 12, 18, 20, 30, 32, 40, 48, 72, 80, 90, 120, 144, 150, 180, 240, 256, 270, 288, 324, 360, 400, 480,
+     486, 600, 750, 864, 900, 960, 1024, 14, 56, 1152]
+Z = [4, 9, 8, 15, 16, 25, 27, 12, 20, 36, 60, 64, 81, 100, 135, 144, 180, 225, 243, 256, 324, 375, 400, 432, 486,
+     576, 625, 729, 768, 810, 900, 1024, 21, 1280]
 
-Y = [4, 6, 10, 18, 32, 40, 48, 80, 90, 144, 150, 256, 270, 324, 400, 480, 600, 750, 960, 1024, 14, 56, 1152]
-Z = [4, 9, 8, 15, 25, 27, 12, 20, 60, 81, 135, 180, 225, 243, 375, 432, 486, 625, 729, 810, 1024, 21, 1280]
+
+@pytest.mark.parametrize("lines", [Y, Z])
+def test_every_radix_in_either_pass(lines):
+    """The plan takes n = r1 r2 with the smallest larger radix r2."""
+    seen = set()
+    for n in lines:
+        plan = next(((n // r, r) for r in RADICES if n % r == 0 and n // r in RADICES and n // r <= r), None)
+        assert (plan is None) == (_lib_tile(n) == 1), n
+        seen |= {(q, r) for q, r in enumerate(plan or ())}
+    assert seen == {(q, r) for q in (0, 1) for r in RADICES}
 
 
+def _lib_tile(n):
+    t = _lib.TileShape()
+    _lib.check(_lib.lib().afid_fft_tile_shape(10, n, 0, 0, C.byref(t)))
+    return t.z_tile
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("nym,nzm", [(y, 9) for y in Y] + [(10, z) for z in Z] + [(150, 135), (64, 96), (32, 45)])
 def test_pressure_solve_line_lengths(ctx, nym, nzm):
     # white noise on a uniform grid of 6 planes: the solve amplifies rounding

@@ -109,7 +109,8 @@ def test_on_chip_solves_match_oracle(ctx, nxm):
     ctx.remove_box(box)
 
 
-@pytest.mark.parametrize("nxm,nym,nzm", [(4, 8, 12), (9, 10, 9), (33, 60, 30), (436, 8, 12), (440, 8, 12)])
+@pytest.mark.parametrize("nxm,nym,nzm", [(4, 8, 12), (8, 10, 9), (9, 10, 9), (16, 12, 10), (17, 12, 10),
+                                         (33, 60, 30), (436, 8, 12), (440, 8, 12)])
 def test_on_chip_pressure_solve_matches_oracle(ctx, nxm, nym, nzm):
     """The x-solve with the modes' columns on chip (up to nxm = 438), over mode
     counts that do not fill the last warp, and one box beyond it."""
@@ -130,12 +131,31 @@ def test_pressure_solve_forms_agree(ctx):
     cfg = cfg_of(40, 64, 30, dt=5e-4, ylen=1.3, zlen=0.9)
     filler = [cfg_of(200, 320, 256, dt=1e-4)]     # two warps per SM: beyond four rounds
     a, b = _boxes(ctx, [cfg])[0], _boxes(ctx, [cfg] + filler)
+    assert ctx.forms([a])["poisson_on_chip"] == 1 and ctx.forms(b)["poisson_on_chip"] == 0
     ctx.step([a], 2)
     ctx.step(b, 2)
     for f in FIELDS:
         assert np.array_equal(a.download(f), b[0].download(f)), f
     for x in [a] + b:
         ctx.remove_box(x)
+
+
+def test_pressure_solve_chunks(ctx):
+    """k_poisson_x marches chunks of 8 planes: one chunk (3 to 8 planes), and every
+    remainder of two and three, give the bits of the solve on chip."""
+    cfgs = [cfg_of(nxm, 10, 9 + nxm % 2, dt=5e-4, ylen=1.3, zlen=0.9) for nxm in range(3, 18)]
+    filler = cfg_of(440, 8, 12, dt=1e-4, istr3=0)     # too tall for the solve on chip
+    alone, batch = _boxes(ctx, cfgs), _boxes(ctx, cfgs + [filler])
+    assert ctx.forms(batch)["poisson_on_chip"] == 0
+    for b in alone:
+        assert ctx.forms([b])["poisson_on_chip"] == 1
+        ctx.step([b], 2)
+    ctx.step(batch, 2)
+    for a, b in zip(alone, batch):
+        for f in FIELDS:
+            assert np.array_equal(a.download(f), b.download(f)), (a.cfg.nxm, f)
+    for b in alone + batch:
+        ctx.remove_box(b)
 
 
 def _check_divergence(box, s, al, dt):
