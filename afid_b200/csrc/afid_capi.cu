@@ -931,7 +931,7 @@ int launch_step(const Batch *bt, cudaStream_t s, Prof *pf = nullptr) {
     int rc = launch_substep(bt, s, ns, pf);
     if (rc) return rc;
   }
-  k_plate_nu<<<dim3(NU_BLOCKS, nb), 256, 0, s>>>(bt->d_boxes, nb, 1);
+  k_plate_nu<true><<<dim3(NU_BLOCKS, nb), 256, 0, s>>>(bt->d_boxes, nb);
   CKL();
   PMARK(pf, AFID_K_PLATE_NU);
   return 0;
@@ -1837,7 +1837,7 @@ int afid_calc_plate_nu(afid_ctx *c, int id, double *nuslow, double *nusupp) {
   if (rc) return rc;
   rc = set_device(c);
   if (rc) return rc;
-  k_plate_nu<<<dim3(NU_BLOCKS, 1), 256, 0, c->stream>>>(hb->d_self, 1, 0);
+  k_plate_nu<false><<<dim3(NU_BLOCKS, 1), 256, 0, c->stream>>>(hb->d_self, 1);
   CKL();
   double part[2 * NU_BLOCKS];
   CK(cudaMemcpyAsync(part, hb->dev.nu_part, sizeof part, cudaMemcpyDeviceToHost, c->stream));
