@@ -1,18 +1,19 @@
 // Pressure Poisson solve of SolvePressureCorrection.F90:35-151 on one GPU:
 //   y: real-to-complex FFT (two real rows packed in one complex line) of dph;
-//   z: complex FFT along kz on tiles of consecutive ky (in place), the tiles
-//      brought in by TMA;
-//   x: one complex tridiagonal per (ky, kz), Thomas in dgttrf/dgttrs order;
+//   z: complex FFT along kz on tiles of consecutive ky (in place);
+//   x: one complex tridiagonal per (ky, kz), Thomas without pivoting on the pivots
+//      of dgttrf's recurrence, tabulated once;
 //   then the inverse z and y transforms, the latter writing dph.
 // The 2DECOMP pencil transposes of the reference disappear: each transform
 // reads its lines directly from the plane-major layout.
 //
-// The FFTs are Stockham auto-sort passes of radix 16, 8, 4, 2, 3, 5 and 7
-// (plans in increasing radix order, e.g. 768 = 3 x 16 x 16), run in place in
-// shared memory on tiles copied in with cp.async; the last pass of the z and
-// inverse-y transforms streams back to global memory.  Twiddles
-// exp(-2 pi i n / N) come from a table computed on the host in extended
-// precision and copied to shared memory by every block.
+// The tile kernels here transform the lines that k_fft2.cuh has no two radices for
+// (a factor of 7, more than 1024 points, and 2, 3, 5, 972 and 1000): Stockham
+// auto-sort passes of radix 16, 8, 4, 2, 3, 5 and 7, the powers of two first (e.g.
+// 1280 = 16 x 16 x 5), run in place in shared memory on tiles brought in by bulk
+// copies (y) and TMA (z); the last pass of the z and inverse-y transforms streams
+// back to global memory.  Twiddles exp(-2 pi i n / N) come from a table computed on
+// the host in extended precision and copied to shared memory by every block.
 #pragma once
 #include "afid_device.cuh"
 

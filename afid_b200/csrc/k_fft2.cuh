@@ -4,17 +4,24 @@
 //
 // A line is two Stockham passes: R2 butterflies of radix R1, one exchange
 // through shared memory, R1 butterflies of radix R2.  A thread holds one
-// butterfly in registers and reads its inputs straight from HBM, all R1 at
-// once, so a tile costs one load latency, one exchange and two barriers; the
-// three or four blocks of an SM are in different phases and cover each other's
-// loads.  HBM traffic bounds the transforms (32 bytes per complex value); below
-// that, what a tile waits for: loads, exchange, barriers.  The tile kernels of
-// k_fft.cuh, which these replace for such lines, make a pass per radix <= 16
-// over a staged tile with two barriers each.  Per step, y forward, z twice and y
-// inverse, tile kernels against these: 75x150x135 0.41 and 0.21 ms, 192x384x384
-// 2.11 and 1.46, 384x768x768 14.7 and 12.1; and against warp-per-line kernels
-// with 8 or 12 values a lane (three passes at 128 points), 64-box ensemble
-// 1.86 and 1.53, 32x32x32 0.123 and 0.103.
+// butterfly in registers with all its inputs in flight at once.  z reads and writes
+// HBM in the butterflies: a tile costs one load latency, one exchange and two
+// barriers.  y forward reads so and goes through shared memory once more, to part
+// the two rows of a line; y inverse stages its lines there first, from
+// coefficients read once (f2_lines_in); both take four barriers.  The four blocks
+// of an SM (three with a radix above 16, two at 960 and 1024 points, whose buffers
+// take 77 and 82 KB; a launch sizes them for its longest lines) are in different phases and
+// cover each other's loads.  HBM traffic bounds the transforms (32 bytes per complex
+// value); below that, what a tile waits for: loads, exchange, barriers.
+//
+// The tile kernels of k_fft.cuh, which these replace for such lines, make a pass per
+// radix <= 16 over a staged tile with two barriers each.  Per step, y forward, z twice
+// and y inverse, tile kernels against these: 75x150x135 0.41 and 0.21 ms, 192x384x384
+// 2.11 and 1.46, 384x768x768 14.7 and 12.1, 16x1024x1024 1.69 and 1.17; and against
+// warp-per-line kernels with 8 or 12 values a lane (three passes at 128 points),
+// 64-box ensemble 1.86 and 1.53, 32x32x32 0.123 and 0.103, but 48 boxes of 64^3
+// 0.73 and 0.82 and of 32^3 0.22 and 0.27: their 33 and 17 ky fill a z tile of 16
+// badly.
 //
 // The exchange stores value r of butterfly j at row r, column j of a
 // R1 x (R2 | 1) array per line: the writes of a pass run along a row, the reads
@@ -111,7 +118,7 @@ __device__ __forceinline__ void f2_dft(double2 (&v)[R]) {
 
 constexpr int F2_T = 128;            // threads per block
 // Radices by class: 0 has both at most 16 (four blocks per SM, 128 registers a
-// thread), 1 the larger one above 16 (three blocks, 168 registers).
+// thread), 1 the larger one above 16 (at most three blocks, 168 registers).
 __host__ __device__ constexpr int f2_blocks(int cls) { return cls ? 3 : 4; }
 // lines per tile: z takes a power of two of neighbouring ky, y any number
 __host__ __device__ __forceinline__ int f2_lines(int r1, int r2, bool z) {

@@ -587,8 +587,9 @@ __global__ void __launch_bounds__(256, 3) k_implicit_bwd(BatchDev bt, int ns) {
   // the LU rows of the three systems, as offsets from one base (seven
   // separate pointers would hold 14 registers across both sweeps)
   const double *__restrict__ cf = B.coef;
-  const int set = ns * (SYS_N * C_N) * nx;      // the substep's set; int offsets: with 64-bit ones the loop spilled
-                                                // (64-box ensemble 1.33 ms per step, 1.24 so)
+  // the substep's set; int offsets: 64-bit ones spilled 84 bytes of stores and 132 of
+  // loads a thread, these 36 and 44 (64-box ensemble 1.33 ms per step, 1.24 so)
+  const int set = ns * (SYS_N * C_N) * nx;
   const auto lu = [&](int sys, int arr, int k) { return __ldg(cf + (set + (sys * C_N + arr) * nx + k)); };
   const double *__restrict__ y0 = B.ybuf[0] + col;
   const double *__restrict__ y1 = B.ybuf[1] + col;
