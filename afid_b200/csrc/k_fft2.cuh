@@ -32,27 +32,59 @@
 
 namespace afid {
 
-// cos and sin of 2 pi p / q at compile time (series on at most pi/4)
-constexpr double f2_series(double x, bool sine) {
-  double term = sine ? x : 1.0, sum = 0.0;
-  double terms[14] = {};
-  for (int n = 0; n < 14; ++n) {
-    terms[n] = term;
-    const int a = 2 * n + (sine ? 2 : 1);
-    term = -term * x * x / ((double)a * (double)(a + 1));
-  }
-  for (int n = 13; n >= 0; --n) sum += terms[n];   // smallest first
-  return sum;
+// cos and sin of 2 pi p / q at compile time, rounded once: the series on at most
+// pi/4 runs in pairs of doubles (Dekker's sums and products), since in doubles a
+// third of the roots came out up to 1.1 units in the last place off.
+struct F2Pair { double hi, lo; };
+constexpr F2Pair f2_sum(double a, double b) {
+  const double s = a + b, t = s - a;
+  return {s, (a - (s - t)) + (b - t)};
 }
-constexpr double F2_2PI = 6.28318530717958647693;
+constexpr F2Pair f2_prod(double a, double b) {
+  const double S = 134217729.0;                  // 2^27 + 1
+  const double p = a * b, ca = S * a, cb = S * b;
+  const double ah = ca - (ca - a), al = a - ah, bh = cb - (cb - b), bl = b - bh;
+  return {p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
+}
+constexpr F2Pair f2_add(F2Pair a, F2Pair b) {
+  const F2Pair s = f2_sum(a.hi, b.hi);
+  return f2_sum(s.hi, s.lo + (a.lo + b.lo));
+}
+constexpr F2Pair f2_mul(F2Pair a, F2Pair b) {
+  const F2Pair p = f2_prod(a.hi, b.hi);
+  return f2_sum(p.hi, p.lo + (a.hi * b.lo + a.lo * b.hi));
+}
+constexpr F2Pair f2_div(F2Pair a, double n) {
+  const double q = a.hi / n;
+  const F2Pair p = f2_prod(q, n);
+  return f2_sum(q, ((a.hi - p.hi) - p.lo + a.lo) / n);
+}
+constexpr double f2_series(F2Pair x, bool sine) {
+  F2Pair term = sine ? x : F2Pair{1.0, 0.0}, sum = term;
+  const F2Pair x2 = f2_mul(x, x);
+  for (int n = 0; n < 13; ++n) {
+    const int a = 2 * n + (sine ? 2 : 1);
+    term = f2_div(f2_mul(term, x2), -(double)a * (double)(a + 1));
+    sum = f2_add(sum, term);
+  }
+  return sum.hi;
+}
+// 2 pi p / q
+constexpr F2Pair f2_angle(int p, int q) {
+  return f2_div(f2_mul(F2Pair{6.283185307179586, 2.4492935982947064e-16}, F2Pair{(double)p, 0.0}), (double)q);
+}
 constexpr double f2_cos(int p, int q) {
   p %= q;
   if (2 * p > q) p = q - p;
   if (4 * p > q) return -f2_cos(q - 2 * p, 2 * q);
-  if (8 * p > q) return f2_series(F2_2PI * (q - 4 * p) / (4.0 * q), true);
-  return f2_series(F2_2PI * p / q, false);
+  if (8 * p > q) return f2_series(f2_angle(q - 4 * p, 4 * q), true);
+  return f2_series(f2_angle(p, q), false);
 }
 constexpr double f2_sin(int p, int q) { return f2_cos((p % q) * 4 + 3 * q, 4 * q); }   // cos(t - pi/2)
+// the worst of a series in doubles
+static_assert(f2_cos(4, 15) == -0.10452846326765347 && f2_cos(7, 25) == -0.18738131458572463 && f2_sin(1, 15) == 0.4067366430758002 &&
+              f2_cos(7, 30) == 0.10452846326765347 && f2_cos(1, 9) == 0.766044443118978 && f2_cos(8, 27) == -0.28680323271109026 &&
+              f2_sin(1, 32) == 0.19509032201612828, "roots of unity");
 
 template <int R>
 struct F2Roots {
@@ -66,7 +98,7 @@ struct F2Roots {
 };
 
 // a (wr + i wi)
-__device__ __forceinline__ double2 f2_mul(double2 a, double wr, double wi) {
+__device__ __forceinline__ double2 f2_mulc(double2 a, double wr, double wi) {
   return make_double2(__fma_rn(a.x, wr, -(a.y * wi)), __fma_rn(a.x, wi, a.y * wr));
 }
 
@@ -88,7 +120,7 @@ __device__ __forceinline__ void f2_comp(double2 (&v)[A * B]) {
     f2_dft<B, SGN>(u);
 #pragma unroll
     for (int k2 = 0; k2 < B; ++k2)
-      y[n1 * B + k2] = n1 * k2 ? f2_mul(u[k2], w.c[n1 * k2 % (A * B)], SGN * w.s[n1 * k2 % (A * B)]) : u[k2];
+      y[n1 * B + k2] = n1 * k2 ? f2_mulc(u[k2], w.c[n1 * k2 % (A * B)], SGN * w.s[n1 * k2 % (A * B)]) : u[k2];
   }
 #pragma unroll
   for (int k2 = 0; k2 < B; ++k2) {
@@ -264,7 +296,7 @@ __device__ __forceinline__ void f2_second(const F2Tile &T, double2 *ex, const do
 #pragma unroll
     for (int r = 1; r < R; ++r) {
       const double2 w = tws[r * T.r1 + j];
-      v[r] = f2_mul(v[r], w.x, SGN > 0 ? -w.y : w.y);
+      v[r] = f2_mulc(v[r], w.x, SGN > 0 ? -w.y : w.y);
     }
     f2_dft<R, SGN>(v);
     if constexpr (KIND == F2_Z) {
