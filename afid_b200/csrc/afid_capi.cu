@@ -91,6 +91,7 @@ struct Batch {
   int nsst = 1;                     // most substeps of its boxes
   int kseg = 0, nseg = 1;           // planes per block and blocks per column tile of divergence and correction
   int diag_kseg = 0, diag_nseg = 1; // and of the diagnostics
+  int full_tiles = 0;               // column tiles of the tallest box's planes that its boxes' work fills
   F2Shape f2[4];                    // two-pass transforms: y and z of classes 0 and 1
   cudaGraphExec_t gexec = nullptr;
   cudaStream_t gstream = nullptr;
@@ -480,10 +481,11 @@ int nsm_of_device() {
 
 // Planes per block of the marches whose planes are independent (divergence,
 // correction, diagnostics), for a set of ``tiles`` column tiles and at most
-// nxm planes: whole columns from ``limit`` tiles on, else segments that give
-// each SM two rounds of its resident blocks.
-void plane_segments(int nsm, int tiles, int nxm, int limit, int *kseg, int *nseg) {
-  const long long n = tiles >= limit ? 1 : std::min(cdiv(4LL * nsm, std::max(tiles, 1)), cdiv(nxm, KC_U));
+// nxm planes, whose work fills ``full`` tiles of nxm planes: whole columns from
+// ``limit`` of those on, else segments that give each SM two rounds of its
+// resident blocks.
+void plane_segments(int nsm, int tiles, int full, int nxm, int limit, int *kseg, int *nseg) {
+  const long long n = full >= limit ? 1 : std::min(cdiv(4LL * nsm, std::max(tiles, 1)), cdiv(nxm, KC_U));
   *kseg = (int)(cdiv(cdiv(nxm, n), KC_U) * KC_U);
   *nseg = (int)cdiv(nxm, *kseg);
 }
@@ -496,7 +498,10 @@ void plane_segments(int nsm, int tiles, int nxm, int limit, int *kseg, int *nseg
 // on 256x192^2 (144 tiles), 0.28 and 0.31 on 128x216^2 (183), 0.36 and 0.33 on
 // 128x240^2 (225); diagnostics with the dt rule 0.052 and 0.074 on 128x150^2 (88),
 // 0.109 and 0.101 on 256x160^2 (100), 0.134 and 0.103 on 256x192^2, 0.21 and 0.12
-// on 256^3 (256).
+// on 256^3 (256).  In a mixed set whole columns take as long as the tallest boxes',
+// so divergence and correction count its tiles by their planes (eight ensemble
+// boxes, 206 tiles, 137 of full height: 1.25 and 1.28 ms per step); the diagnostics
+// gain nothing by it.
 int column_limit(int nsm) { return 4 * nsm / 3; }
 int diag_limit(int nsm) { return 2 * nsm / 3; }
 
@@ -511,22 +516,25 @@ int diag_limit(int nsm) { return 2 * nsm / 3; }
 // against on chip: 100x180^2 (23) 0.63 and 0.67 ms, 160x192^2 (31) 0.98 and 1.22,
 // 256x160^2 (32) 1.49 and 2.05, 400x192^2 (47) 2.36 and 4.31; below it, the column
 // kernels timed before their divisions went, 160^3 (22) 1.04 and 0.95, 256x128^2
-// (21) 1.60 and 1.35.
+// (21) 1.60 and 1.35.  Blocks count by their planes, as in plane_segments (seven
+// ensemble boxes, 142 tiles, 23 by blocks and 15 by planes: a step takes 0.95 ms on
+// chip and 1.03).
 // Boxes too tall for a block's shared memory (nxm > 401) keep the column
 // kernels.  Results do not depend on the choice.  Returns the shared memory of
 // the k_implicit_cols launch.
 // A half of a split set does as the set would whole.
 size_t choose_on_chip(int nsm, std::vector<BoxDev> &devs, const Batch *whole) {
-  long long tiles = 0, blocks = 0;
+  long long tiles = 0, planes = 0, nxm = 1;   // planes of the blocks, and of the tallest box on chip
   size_t smem = 0;
   for (const BoxDev &d : devs) {
     tiles += cdiv(d.plane, 256);
     if (ks_bytes(d.nxm) > ON_CHIP_SMEM) continue;
-    blocks += 2 * cdiv(d.plane, KS_COLS);
+    planes += 2 * cdiv(d.plane, KS_COLS) * d.nxm;
+    nxm = std::max<long long>(nxm, d.nxm);
     smem = std::max(smem, (size_t)ks_bytes(d.nxm));
   }
   const long long fit = SM_SMEM / (long long)(smem + 1024);
-  const bool on = whole ? whole->smem_ks > 0 : tiles < nsm && blocks * (fit + 2) < 22LL * nsm * fit;
+  const bool on = whole ? whole->smem_ks > 0 : tiles < nsm && planes * (fit + 2) < 22LL * nsm * fit * nxm;
   for (BoxDev &d : devs) d.on_chip = on && ks_bytes(d.nxm) <= ON_CHIP_SMEM;
   return on ? smem : 0;
 }
@@ -629,8 +637,12 @@ int get_batch(afid_ctx *c, const int *ids, int n, Batch **out, const Batch *whol
   for (const BoxDev &d : devs) bt->nsst = std::max(bt->nsst, d.nsst);
   const int *total = whole ? whole->total : bt->total;   // of the launches that share the device
   bt->smem_px = px_cols_smem(nsm, bt->total[FAM_PXS], devs[0].nxm, whole != nullptr);
-  plane_segments(nsm, total[FAM_COL], devs[0].nxm, column_limit(nsm), &bt->kseg, &bt->nseg);
-  plane_segments(nsm, total[FAM_DIAG], devs[0].nxm, diag_limit(nsm), &bt->diag_kseg, &bt->diag_nseg);
+  long long planes = 0;
+  for (const BoxDev &d : devs) planes += tiles_of(d, FAM_COL) * d.nxm;
+  bt->full_tiles = (int)cdiv(planes, devs[0].nxm);
+  plane_segments(nsm, total[FAM_COL], whole ? whole->full_tiles : bt->full_tiles, devs[0].nxm, column_limit(nsm),
+                 &bt->kseg, &bt->nseg);
+  plane_segments(nsm, total[FAM_DIAG], total[FAM_DIAG], devs[0].nxm, diag_limit(nsm), &bt->diag_kseg, &bt->diag_nseg);
   k1s_segments(nsm, total[FAM_K1S], devs[0].nxm, &bt->k1s_seg, &bt->k1s_nseg);
   off.insert(off.end(), pos.begin(), pos.end());   // the positions follow the tile tables
   if (cudaMalloc(&bt->d_boxes, sizeof(BoxDev) * n) != cudaSuccess ||

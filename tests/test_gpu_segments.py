@@ -94,6 +94,23 @@ def test_segments_where_they_gain(ctx, n, column, diag):
     ctx.remove_box(box)
 
 
+def test_forms_of_mixed_sets(ctx):
+    """Column kernels take as long as the tallest box's columns, so a set of mostly low
+    boxes keeps the forms that spread its work: segments at 208 tiles, on-chip
+    solves at 142; a set of equal heights does not."""
+    low = [ctx.add_box(cfg_of(32, 128, 128, dt=1e-5)) for _ in range(3)]
+    tall = [ctx.add_box(cfg_of(96, 64, 64, dt=1e-5))]
+    assert ctx.forms(low + tall)["column_segments"] > 1
+    same = [ctx.add_box(cfg_of(32, 128, 128, dt=1e-5))]
+    assert ctx.forms(low + same)["column_segments"] == 1
+    high = [ctx.add_box(cfg_of(96, 16, 16, dt=1e-5)) for _ in range(14)]
+    flat = [ctx.add_box(cfg_of(96, 128, 128, dt=1e-5)) for _ in range(2)]
+    assert ctx.forms(low[:2] + high)["implicit_on_chip"] == 1
+    assert ctx.forms(flat + high)["implicit_on_chip"] == 0
+    for b in low + tall + same + high + flat:
+        ctx.remove_box(b)
+
+
 @pytest.mark.parametrize("nxm", [4, 9, 33, 400, 404])
 def test_on_chip_solves_match_oracle(ctx, nxm):
     """nxm = 400 is near the tallest on-chip column, 404 is beyond it."""
